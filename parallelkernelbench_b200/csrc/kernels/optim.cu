@@ -11,6 +11,7 @@
 // per-tensor delayed scaling (reference: reference/47_fsdp_step_e2e.py:49-65,
 // reference/52_fp8_reduce_scatter_grads.py:26-41, reference/53_fp8_allgather_params.py:26-39).
 #include <cuda_fp8.h>
+#include <math.h>
 
 #include "pkb/api.h"
 #include "pkb/host.h"
@@ -29,18 +30,25 @@ struct FsdpAdamArgs {
   uint8_t* q_out;          // [n] new weights as e4m3
   float* s_out;            // [n / 128]
   __nv_bfloat16* p_bf16;   // optional bf16 copy of the new weights
-  float lr, beta1, beta2, eps, weight_decay, grad_scale, bias_c1, bias_c2;
+  float beta1, beta2, eps, grad_scale;
+  float decay;             // 1 - lr * weight_decay
+  float step_size;         // lr / (1 - beta1^step)
+  float inv_sqrt_c2;       // 1 / sqrt(1 - beta2^step)
 };
 
-__device__ __forceinline__ float e4m3_to_float(uint32_t byte) {
-  __half_raw h = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)byte, __NV_E4M3);
-  return __half2float(*reinterpret_cast<__half*>(&h));
+__device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t two_bytes) {
+  __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)two_bytes, __NV_E4M3);
+  return __half22float2(*reinterpret_cast<__half2*>(&h));
 }
 
 // One 128-element block per warp iteration, four elements per lane: every access of a warp is coalesced and the kernel runs
 // at full occupancy (40 registers). Two wider forms were measured and dropped: 16 consecutive elements per thread (strided
 // warp accesses, 307 us against 292 us on the 8-rank profile case) and four blocks per warp iteration with all loads issued
 // first (128 registers, a quarter of the occupancy, 585 us).
+// 26 bytes move per element at W = 1. What bounded the first form (3.8 TB/s) was not memory but the division sequences: three
+// and a square root per element, two more per lane and block. The bias corrections are now folded into two constants (one
+// division and the root remain), amax / 448 is a product with a correction, and the e4m3 bytes are converted in pairs.
+// Measured over the 961 M parameters of two 8B-shaped layers and their embedding: 6.64 ms before, 4.96 ms now.
 __global__ void __launch_bounds__(256) fsdp_adamw_fp8_kernel(const FsdpAdamArgs a) {
   const int lane = threadIdx.x & 31;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -48,42 +56,41 @@ __global__ void __launch_bounds__(256) fsdp_adamw_fp8_kernel(const FsdpAdamArgs 
   const long long nb = a.n / 128;
   for (long long b = warp; b < nb; b += nwarps) {
     const long long i0 = b * 128 + lane * 4;
+    // master weights and moments move as 16-byte vectors (i0 is a multiple of 4 elements); read and written once: streaming
+    const float4 p4 = __ldcs(reinterpret_cast<const float4*>(a.p + i0));
+    const float4 m4 = __ldcs(reinterpret_cast<const float4*>(a.m + i0));
+    const float4 v4 = __ldcs(reinterpret_cast<const float4*>(a.v + i0));
     float g[4] = {0.f, 0.f, 0.f, 0.f};
     for (int w = 0; w < a.W; ++w) {
       const uint32_t packed = *reinterpret_cast<const uint32_t*>(a.payload + (long long)w * a.n + i0);
       const float s = a.scales[(long long)w * nb + b];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) g[j] += e4m3_to_float((packed >> (8 * j)) & 0xffu) * s;
+      const float2 lo = e4m3x2_to_float2(packed & 0xffffu), hi = e4m3x2_to_float2(packed >> 16);
+      g[0] += lo.x * s; g[1] += lo.y * s; g[2] += hi.x * s; g[3] += hi.y * s;
     }
     float wnew[4];
     float amax = 0.f;
-    // master weights and moments move as 16-byte vectors (i0 is a multiple of 4 elements)
-    const float4 p4 = *reinterpret_cast<const float4*>(a.p + i0);
-    const float4 m4 = *reinterpret_cast<const float4*>(a.m + i0);
-    const float4 v4 = *reinterpret_cast<const float4*>(a.v + i0);
     const float pin[4] = {p4.x, p4.y, p4.z, p4.w}, min_[4] = {m4.x, m4.y, m4.z, m4.w}, vin[4] = {v4.x, v4.y, v4.z, v4.w};
     float mo[4], vo[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float grad = g[j] * a.grad_scale;
-      float w = pin[j] * (1.0f - a.lr * a.weight_decay);
       const float mi = a.beta1 * min_[j] + (1.0f - a.beta1) * grad;
       const float vi = a.beta2 * vin[j] + (1.0f - a.beta2) * grad * grad;
-      w -= a.lr * (mi / a.bias_c1) / (sqrtf(vi / a.bias_c2) + a.eps);
+      const float w = pin[j] * a.decay - a.step_size * mi / (sqrtf(vi) * a.inv_sqrt_c2 + a.eps);
       mo[j] = mi; vo[j] = vi;
       wnew[j] = w;
       amax = fmaxf(amax, fabsf(w));
     }
-    *reinterpret_cast<float4*>(a.p + i0) = make_float4(wnew[0], wnew[1], wnew[2], wnew[3]);
-    *reinterpret_cast<float4*>(a.m + i0) = make_float4(mo[0], mo[1], mo[2], mo[3]);
-    *reinterpret_cast<float4*>(a.v + i0) = make_float4(vo[0], vo[1], vo[2], vo[3]);
+    __stcs(reinterpret_cast<float4*>(a.p + i0), make_float4(wnew[0], wnew[1], wnew[2], wnew[3]));
+    __stcs(reinterpret_cast<float4*>(a.m + i0), make_float4(mo[0], mo[1], mo[2], mo[3]));
+    __stcs(reinterpret_cast<float4*>(a.v + i0), make_float4(vo[0], vo[1], vo[2], vo[3]));
     if (a.p_bf16) {
       *reinterpret_cast<uint2*>(a.p_bf16 + i0) = make_uint2(pack_bf16x2(wnew[0], wnew[1]), pack_bf16x2(wnew[2], wnew[3]));
     }
     amax = warp_max(amax);
-    float s = amax / 448.0f;
+    float s = div_rn_by(amax, 448.0f, 1.0f / 448.0f);
     if (s == 0.f) s = 1.0f;
-    const float inv = 1.0f / s;
+    const float inv = __frcp_rn(s);
     __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(wnew[0] * inv, wnew[1] * inv), __NV_SATFINITE, __NV_E4M3);
     __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(wnew[2] * inv, wnew[3] * inv), __NV_SATFINITE, __NV_E4M3);
     *reinterpret_cast<uint32_t*>(a.q_out + i0) = (uint32_t)lo | ((uint32_t)hi << 16);
@@ -102,8 +109,9 @@ extern "C" int pkb_fsdp_adamw_fp8(const void* payload, const void* scales, int W
   if (n == 0) return kApiOk;
   FsdpAdamArgs a{static_cast<const uint8_t*>(payload), static_cast<const float*>(scales), W, n,
                  static_cast<float*>(p), static_cast<float*>(m), static_cast<float*>(v), static_cast<uint8_t*>(q_out),
-                 static_cast<float*>(s_out), static_cast<__nv_bfloat16*>(p_bf16), lr, beta1, beta2, eps, weight_decay,
-                 grad_scale, 1.0f - powf(beta1, (float)step), 1.0f - powf(beta2, (float)step)};
+                 static_cast<float*>(s_out), static_cast<__nv_bfloat16*>(p_bf16), beta1, beta2, eps, grad_scale,
+                 1.0f - lr * weight_decay, (float)(lr / (1.0 - pow((double)beta1, (double)step))),
+                 (float)(1.0 / sqrt(1.0 - pow((double)beta2, (double)step)))};
   PKB_CHECK_ARG((((uintptr_t)payload | (uintptr_t)p | (uintptr_t)m | (uintptr_t)v | (uintptr_t)q_out | (uintptr_t)p_bf16) & 15) == 0,
                 "buffers must be 16-byte aligned");
   long long blocks = (n / 128 * 32 + 255) / 256;

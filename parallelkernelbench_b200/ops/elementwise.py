@@ -168,10 +168,13 @@ def rmsnorm_bwd(x: torch.Tensor, gamma: torch.Tensor, dy: torch.Tensor, eps: flo
     rows, H = x.shape
     xc, dyc, gc = x.contiguous(), dy.contiguous(), gamma.reshape(-1).contiguous()
     dx = torch.empty_like(xc)
-    dg = torch.zeros(H, dtype=torch.float32, device=x.device)
-    nv.check(nv.cuda_lib().pkb_rmsnorm_bwd(nv.ptr(xc), nv.ptr(gc), nv.ptr(dyc), nv.ptr(dx), nv.ptr(dg), rows, H, nv.c_float(eps),
-                                           nv.current_stream()), "pkb_rmsnorm_bwd")
-    nv.count_launch()
+    lib = nv.cuda_lib()
+    nblk = lib.pkb_rmsnorm_bwd_partials(rows, H)
+    dg = torch.empty(H, dtype=torch.float32, device=x.device) if nblk else torch.zeros(H, dtype=torch.float32, device=x.device)
+    part = torch.empty((nblk, H), dtype=torch.float32, device=x.device) if nblk else None
+    nv.check(lib.pkb_rmsnorm_bwd(nv.ptr(xc), nv.ptr(gc), nv.ptr(dyc), None, nv.ptr(dx), nv.ptr(dg), None, nv.ptr(part), rows, H,
+                                 nv.c_float(eps), nv.current_stream()), "pkb_rmsnorm_bwd")
+    nv.count_launch(2 if nblk else 1)
     return dx, dg
 
 

@@ -113,6 +113,13 @@ def current_stream() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def raw_stream(t) -> int:
+    """The current stream of the tensor's device as an integer, for functions with declared argument types."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
+
+
 def read_status() -> list[int]:
     buf = (ctypes.c_uint32 * 16)()
     check(cuda_lib().pkb_status_read(buf), "pkb_status_read")

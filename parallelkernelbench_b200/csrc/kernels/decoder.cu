@@ -1,0 +1,233 @@
+// One decoder layer, forward and backward, as a sequence of this library's launches issued by one native call each.
+//
+// The launches of a layer are known from its shape alone, so the host side needs no tape: the forward writes what the backward
+// will read into one `saved` buffer, the backward writes every weight gradient into its place of the layer's flat gradient
+// buffer (no concatenation afterwards). Issued from Python through an autograd tape, a layer of the small configuration
+// (hidden 512, 256 tokens) cost about 1.2 ms of host time for 0.25 ms of device time.
+//
+// Layer: h = rms(x) ; q, k, v = rope(h Wqkv^T) ; x1 = x + attention(q, k, v) Wo^T ; out = x1 + swiglu(rms(x1) Wgu^T) Wdown^T
+// Parameters lie flat in the order Wqkv, Wo, Wgu, Wdown, norm1, norm2 (bf16).
+#include "pkb/api.h"
+#include "pkb/attention_api.h"
+#include "pkb/decoder_api.h"
+#include "pkb/host.h"
+
+using namespace pkb;
+
+extern "C" {
+int pkb_gemm_bf16_pair(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N, int K,
+                       const void* bias, float alpha, int epilogue, int out_f32, int num_ctas, void* stream);
+int pkb_gemm_bf16_bkn(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N, int K,
+                      float alpha, int epilogue, int out_f32, void* stream);
+int pkb_gemm_bf16_tn(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N, int K,
+                     float alpha, int out_f32, void* stream);
+int pkb_add_rmsnorm_bf16(const void* x, const void* y, const void* gamma, void* sum, void* out, int rows, int cols, float eps, void* stream);
+int pkb_swiglu_fwd(const void* gu, void* a, long long rows, int F, void* stream);
+int pkb_swiglu_bwd(const void* gu, const void* da, void* dgu, long long rows, int F, void* stream);
+int pkb_rmsnorm_bwd_partials(int rows, int H);
+int pkb_rmsnorm_bwd(const void* x, const void* gamma, const void* dy, const void* res, void* dx, void* dgamma, void* dgamma_bf16,
+                    void* partial, int rows, int H, float eps, void* stream);
+int pkb_qkv_rope_split(const void* qkv, const void* cos_t, const void* sin_t, void* q, void* k, void* v, int tokens, int hq, int hkv,
+                       int d, void* stream);
+int pkb_qkv_rope_merge(const void* dq, const void* dk, const void* dv, const void* cos_t, const void* sin_t, void* dqkv, int tokens,
+                       int hq, int hkv, int d, void* stream);
+int pkb_add_bf16(const void* a, const void* b, void* out, long long n, void* stream);
+int pkb_flash_attn_fwd(const pkb_attn_desc* desc, const void* q, const void* k, const void* v, void* out, void* lse, void* stream);
+int pkb_flash_attn_bwd(const pkb_attn_desc* desc, const void* q, const void* k, const void* v, const void* o, const void* dout,
+                       const void* lse, void* delta_scratch, void* lse2_scratch, void* dq, void* dk, void* dv, void* stream);
+}
+
+namespace {
+
+struct Carve {          // hands out 256-byte aligned pieces of a buffer; with a null base it only counts
+  uint8_t* base;
+  long long used = 0;
+  void* take(long long bytes) {
+    void* p = base ? base + used : nullptr;
+    used += (bytes + 255) / 256 * 256;
+    return p;
+  }
+};
+
+struct Saved {
+  void *h, *q, *k, *v, *att, *lse, *x1, *h2, *gu, *a;
+  void layout(const pkb_layer_desc& L, Carve& c) {
+    const long long S = L.tokens, qd = (long long)L.hq * L.head_dim, kd = (long long)L.hkv * L.head_dim;
+    h = c.take(S * L.hidden * 2);
+    q = c.take(S * qd * 2);
+    k = c.take(S * kd * 2);
+    v = c.take(S * kd * 2);
+    att = c.take(S * qd * 2);
+    lse = c.take(S * L.hq * 4);
+    x1 = c.take(S * L.hidden * 2);
+    h2 = c.take(S * L.hidden * 2);
+    gu = c.take(S * 2 * L.ffn * 2);
+    a = c.take(S * L.ffn * 2);
+  }
+};
+
+struct FwdScratch {
+  void *qkv, *o, *down;
+  void layout(const pkb_layer_desc& L, Carve& c) {
+    const long long S = L.tokens;
+    qkv = c.take(S * (L.hq + 2ll * L.hkv) * L.head_dim * 2);
+    o = c.take(S * L.hidden * 2);
+    down = o;           // consumed by the fused add before the MLP starts
+  }
+};
+
+struct BwdScratch {
+  void *da, *dgu, *dh2, *dx1, *datt, *delta, *lse2, *dqkv32, *dqkv, *dh, *partial;
+  long long dq_elems, dk_elems;
+  void layout(const pkb_layer_desc& L, Carve& c) {
+    const long long S = L.tokens, qd = (long long)L.hq * L.head_dim, kd = (long long)L.hkv * L.head_dim;
+    da = c.take(S * L.ffn * 2);
+    dgu = c.take(S * 2 * L.ffn * 2);
+    dh2 = c.take(S * L.hidden * 2);
+    dx1 = c.take(S * L.hidden * 2);
+    datt = c.take(S * qd * 2);
+    delta = c.take(S * L.hq * 4);
+    lse2 = c.take(S * L.hq * 4);
+    dq_elems = S * qd;
+    dk_elems = S * kd;
+    dqkv32 = c.take((dq_elems + 2 * dk_elems) * 4);      // dq, dk, dv in one piece: one fill
+    dqkv = c.take(S * (qd + 2 * kd) * 2);
+    dh = c.take(S * L.hidden * 2);
+    partial = c.take((long long)pkb_rmsnorm_bwd_partials(L.tokens, L.hidden) * L.hidden * 4);
+  }
+};
+
+struct Params {          // element offsets into the flat buffer
+  long long wqkv, wo, wgu, wdown, norm1, norm2, total;
+  explicit Params(const pkb_layer_desc& L) {
+    const long long H = L.hidden, qd = (long long)L.hq * L.head_dim, kd = (long long)L.hkv * L.head_dim;
+    wqkv = 0;
+    wo = wqkv + (qd + 2 * kd) * H;
+    wgu = wo + H * qd;
+    wdown = wgu + 2ll * L.ffn * H;
+    norm1 = wdown + H * (long long)L.ffn;
+    norm2 = norm1 + H;
+    total = norm2 + H;
+  }
+};
+
+inline const void* at(const void* base, long long elem) { return static_cast<const uint8_t*>(base) + elem * 2; }
+inline void* at(void* base, long long elem) { return static_cast<uint8_t*>(base) + elem * 2; }
+
+// y[M, N] = x[M, K] w[N, K]^T
+int linear(const void* x, const void* w, void* y, int M, int N, int K, void* stream) {
+  if (M >= 512 && N >= 256) return pkb_gemm_bf16_pair(x, K, w, K, y, N, M, N, K, nullptr, 1.0f, 0, 0, 0, stream);
+  return pkb_gemm_bf16(x, K, w, K, y, N, M, N, K, nullptr, 1.0f, 0, 0, 0, 0, stream);
+}
+// dx[M, K] = dy[M, N] w[N, K]
+int linear_dx(const void* dy, const void* w, void* dx, int M, int N, int K, void* stream) {
+  return pkb_gemm_bf16_bkn(dy, N, w, K, dx, K, M, K, N, 1.0f, 0, 0, stream);
+}
+// dw[N, K] = dy[M, N]^T x[M, K]
+int linear_dw(const void* dy, const void* x, void* dw, int M, int N, int K, void* stream) {
+  return pkb_gemm_bf16_tn(dy, N, x, K, dw, K, N, K, M, 1.0f, 0, stream);
+}
+
+void attn_desc(const pkb_layer_desc& L, pkb_attn_desc& d) {
+  d = pkb_attn_desc{};
+  d.batch = 1;
+  d.sq = d.skv = L.tokens;
+  d.hq = L.hq;
+  d.hkv = L.hkv;
+  d.head_dim = L.head_dim;
+  d.causal = 1;
+  d.scale = L.scale;
+  d.q_seg_rows = L.tokens;
+  d.num_q_segs = 1;
+  d.num_kv_segs = 1;
+  d.kv_seg_len[0] = L.tokens;
+}
+
+int check(const pkb_layer_desc* L) {
+  PKB_CHECK_ARG(L != nullptr && L->tokens > 0 && L->hidden > 0 && L->ffn > 0 && L->hq > 0 && L->hkv > 0 && L->hq % L->hkv == 0, "bad layer shape");
+  PKB_CHECK_ARG(L->hidden % 8 == 0 && L->ffn % 8 == 0 && L->hidden <= 8192, "hidden and ffn must be multiples of 8, hidden at most 8192");
+  PKB_CHECK_ARG(L->head_dim == 64 || L->head_dim == 128, "head_dim must be 64 or 128");
+  return kApiOk;
+}
+
+}  // namespace
+
+#define PKB_TRY(call)       \
+  do {                      \
+    const int _rc = (call); \
+    if (_rc) return _rc;    \
+  } while (0)
+
+extern "C" int pkb_decoder_layer_sizes(const pkb_layer_desc* L, long long* saved, long long* fwd_scratch, long long* bwd_scratch) {
+  PKB_TRY(check(L));
+  Carve c0{nullptr}, c1{nullptr}, c2{nullptr};
+  Saved s;
+  s.layout(*L, c0);
+  FwdScratch f;
+  f.layout(*L, c1);
+  BwdScratch b;
+  b.layout(*L, c2);
+  *saved = c0.used;
+  *fwd_scratch = c1.used;
+  *bwd_scratch = c2.used;
+  return kApiOk;
+}
+
+extern "C" int pkb_decoder_layer_fwd(const pkb_layer_desc* L, const void* x, const void* params, const void* cos_t, const void* sin_t,
+                                     void* out, void* saved, void* scratch, void* st) {
+  PKB_TRY(check(L));
+  const int S = L->tokens, H = L->hidden, F = L->ffn, d = L->head_dim;
+  const int QD = L->hq * d, QKV = (L->hq + 2 * L->hkv) * d;
+  const Params p(*L);
+  Carve cs{static_cast<uint8_t*>(saved)}, cf{static_cast<uint8_t*>(scratch)};
+  Saved s;
+  s.layout(*L, cs);
+  FwdScratch f;
+  f.layout(*L, cf);
+  PKB_TRY(pkb_rmsnorm_bf16(x, at(params, p.norm1), s.h, S, H, L->eps, st));
+  PKB_TRY(linear(s.h, at(params, p.wqkv), f.qkv, S, QKV, H, st));
+  PKB_TRY(pkb_qkv_rope_split(f.qkv, cos_t, sin_t, s.q, s.k, s.v, S, L->hq, L->hkv, d, st));
+  pkb_attn_desc ad;
+  attn_desc(*L, ad);
+  PKB_TRY(pkb_flash_attn_fwd(&ad, s.q, s.k, s.v, s.att, s.lse, st));
+  PKB_TRY(linear(s.att, at(params, p.wo), f.o, S, H, QD, st));
+  PKB_TRY(pkb_add_rmsnorm_bf16(x, f.o, at(params, p.norm2), s.x1, s.h2, S, H, L->eps, st));
+  PKB_TRY(linear(s.h2, at(params, p.wgu), s.gu, S, 2 * F, H, st));
+  PKB_TRY(pkb_swiglu_fwd(s.gu, s.a, S, F, st));
+  PKB_TRY(linear(s.a, at(params, p.wdown), f.down, S, H, F, st));
+  return pkb_add_bf16(s.x1, f.down, out, (long long)S * H, st);
+}
+
+extern "C" int pkb_decoder_layer_bwd(const pkb_layer_desc* L, const void* x, const void* params, const void* cos_t, const void* sin_t,
+                                     const void* saved, const void* dout, void* dx, void* dparams, void* scratch, void* st) {
+  PKB_TRY(check(L));
+  const int S = L->tokens, H = L->hidden, F = L->ffn, d = L->head_dim;
+  const int QD = L->hq * d, QKV = (L->hq + 2 * L->hkv) * d;
+  const Params p(*L);
+  Carve cs{static_cast<uint8_t*>(const_cast<void*>(saved))}, cb{static_cast<uint8_t*>(scratch)};
+  Saved s;
+  s.layout(*L, cs);
+  BwdScratch b;
+  b.layout(*L, cb);
+  // MLP
+  PKB_TRY(linear_dx(dout, at(params, p.wdown), b.da, S, H, F, st));
+  PKB_TRY(linear_dw(dout, s.a, at(dparams, p.wdown), S, H, F, st));
+  PKB_TRY(pkb_swiglu_bwd(s.gu, b.da, b.dgu, S, F, st));
+  PKB_TRY(linear_dx(b.dgu, at(params, p.wgu), b.dh2, S, 2 * F, H, st));
+  PKB_TRY(linear_dw(b.dgu, s.h2, at(dparams, p.wgu), S, 2 * F, H, st));
+  PKB_TRY(pkb_rmsnorm_bwd(s.x1, at(params, p.norm2), b.dh2, dout, b.dx1, nullptr, at(dparams, p.norm2), b.partial, S, H, L->eps, st));
+  // attention
+  PKB_TRY(linear_dx(b.dx1, at(params, p.wo), b.datt, S, H, QD, st));
+  PKB_TRY(linear_dw(b.dx1, s.att, at(dparams, p.wo), S, H, QD, st));
+  pkb_attn_desc ad;
+  attn_desc(*L, ad);
+  float* dq = static_cast<float*>(b.dqkv32);
+  float* dk = dq + b.dq_elems;
+  float* dv = dk + b.dk_elems;
+  PKB_CHECK_CUDA(cudaMemsetAsync(dq, 0, (size_t)(b.dq_elems + 2 * b.dk_elems) * 4, static_cast<cudaStream_t>(st)));
+  PKB_TRY(pkb_flash_attn_bwd(&ad, s.q, s.k, s.v, s.att, b.datt, s.lse, b.delta, b.lse2, dq, dk, dv, st));
+  PKB_TRY(pkb_qkv_rope_merge(dq, dk, dv, cos_t, sin_t, b.dqkv, S, L->hq, L->hkv, d, st));
+  PKB_TRY(linear_dx(b.dqkv, at(params, p.wqkv), b.dh, S, QKV, H, st));
+  PKB_TRY(linear_dw(b.dqkv, s.h, at(dparams, p.wqkv), S, QKV, H, st));
+  return pkb_rmsnorm_bwd(x, at(params, p.norm1), b.dh, b.dx1, dx, nullptr, at(dparams, p.norm1), b.partial, S, H, L->eps, st);
+}

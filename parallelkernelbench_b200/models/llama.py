@@ -7,7 +7,8 @@ Two implementations share this file's structure:
   MN-major-B kernel, weight gradient through the transposed-A kernel - no transposed copies),
   flash-attention forward, RMSNorm, RoPE and cross-entropy on our kernels, parameters gathered as
   e4m3 bytes + 1x128 scales over the symmetric heap, gradients sent as fp8 slices and reduced inside
-  the fused dequant-sum + AdamW + requantise kernel.
+  the fused dequant-sum + AdamW + requantise kernel. No autograd tape: a layer's forward and backward are
+  one native call each (``ops.decoder.DecoderLayer``).
 * ``impl="torch"``  the PyTorch + NCCL + cuBLAS baseline of the same step (bf16 all-gather,
   reduce-scatter, library attention, torch AdamW arithmetic).
 
@@ -58,121 +59,6 @@ class LlamaConfig:
         return sum(a * b for _, (a, b) in self.layer_shapes())
 
 
-# =================================================================================================
-# autograd functions over our kernels
-# =================================================================================================
-class _Linear(torch.autograd.Function):
-    """y = x @ w.T ; dx = dy @ w (w read as an MN-major operand) ; dw = dy.T @ x (transposed-A kernel)."""
-
-    @staticmethod
-    def forward(ctx, x, w):
-        from ..ops import gemm_bf16
-
-        ctx.save_for_backward(x, w)
-        return gemm_bf16(x, w)
-
-    @staticmethod
-    def backward(ctx, dy):
-        from ..ops import gemm_bf16_kn, gemm_bf16_tn
-
-        x, w = ctx.saved_tensors
-        dy = dy.contiguous()
-        return gemm_bf16_kn(dy, w), gemm_bf16_tn(dy, x)
-
-
-class _RMSNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, gamma, eps):
-        from ..ops import rmsnorm
-
-        ctx.save_for_backward(x, gamma)
-        ctx.eps = eps
-        return rmsnorm(x, gamma.reshape(-1), eps)
-
-    @staticmethod
-    def backward(ctx, dy):
-        from ..ops import rmsnorm_bwd
-
-        x, gamma = ctx.saved_tensors
-        dx, dg = rmsnorm_bwd(x, gamma, dy.contiguous(), ctx.eps)
-        return dx, dg.to(gamma.dtype).reshape(gamma.shape), None
-
-
-class _SwiGLU(torch.autograd.Function):
-    """``silu(gate) * up`` over the packed [tokens, 2 * ffn] projection, forward and backward in one pass each."""
-
-    @staticmethod
-    def forward(ctx, gu):
-        from ..ops import swiglu_fwd
-
-        ctx.save_for_backward(gu)
-        return swiglu_fwd(gu)
-
-    @staticmethod
-    def backward(ctx, da):
-        from ..ops import swiglu_bwd
-
-        (gu,) = ctx.saved_tensors
-        return swiglu_bwd(gu, da.contiguous())
-
-
-class _Rope(torch.autograd.Function):
-    """Rotate-half RoPE; the backward is the inverse rotation (same kernel with the sine negated)."""
-
-    @staticmethod
-    def forward(ctx, x, cos, sin):
-        from ..ops import rope
-
-        ctx.save_for_backward(cos, sin)
-        return rope(x, cos, sin)
-
-    @staticmethod
-    def backward(ctx, dy):
-        from ..ops import rope
-
-        cos, sin = ctx.saved_tensors
-        return rope(dy.contiguous(), cos, -sin), None, None
-
-
-class _SplitQKV(torch.autograd.Function):
-    """[S, (Hq + 2 Hkv) d] -> q [1, S, Hq, d], k, v [1, S, Hkv, d] (contiguous). The backward is one concatenation; autograd's
-    own slice backward would zero-fill three projection-sized tensors and add them up."""
-
-    @staticmethod
-    def forward(ctx, qkv, hq, hkv, d):
-        S = qkv.shape[0]
-        ctx.dims = (hq, hkv, d)
-        q = qkv[:, :hq * d].reshape(1, S, hq, d).contiguous()
-        k = qkv[:, hq * d:(hq + hkv) * d].reshape(1, S, hkv, d).contiguous()
-        v = qkv[:, (hq + hkv) * d:].reshape(1, S, hkv, d).contiguous()
-        return q, k, v
-
-    @staticmethod
-    def backward(ctx, dq, dk, dv):
-        hq, hkv, d = ctx.dims
-        S = dq.shape[1]
-        return torch.cat([dq.reshape(S, hq * d), dk.reshape(S, hkv * d), dv.reshape(S, hkv * d)], dim=1), None, None, None
-
-
-class _FlashAttention(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, scale):
-        from ..ops.attention import flash_attn_fwd
-
-        out, lse = flash_attn_fwd(q, k, v, causal=True, scale=scale)
-        ctx.save_for_backward(q, k, v, out, lse)
-        ctx.scale = scale
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        from ..ops.attention import flash_attn_bwd
-
-        q, k, v, out, lse = ctx.saved_tensors
-        dq, dk, dv = flash_attn_bwd(q, k, v, out, lse, dout.contiguous(), causal=True, scale=ctx.scale)
-        return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), None
-
-
 def rope_tables(cfg: LlamaConfig, device, dtype=torch.bfloat16):
     d = cfg.head_dim
     inv = 1.0 / (cfg.rope_theta ** (torch.arange(0, d, 2, device=device, dtype=torch.float32) / d))
@@ -181,7 +67,7 @@ def rope_tables(cfg: LlamaConfig, device, dtype=torch.bfloat16):
 
 
 # =================================================================================================
-# one decoder layer, either on our kernels or on PyTorch library ops
+# one decoder layer on PyTorch library ops (impl="torch"); impl="ours" is ops.decoder.DecoderLayer
 # =================================================================================================
 def _rot_half(x, cos, sin):
     h = x.shape[-1] // 2
@@ -193,33 +79,19 @@ def _rms_torch(x, g, eps):
     return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps) * g.float().reshape(-1)).to(x.dtype)
 
 
-def layer_forward(cfg: LlamaConfig, p: dict, x: torch.Tensor, cos, sin, impl: str) -> torch.Tensor:
+def layer_forward(cfg: LlamaConfig, p: dict, x: torch.Tensor, cos, sin) -> torch.Tensor:
     """``x`` is ``[S, hidden]`` (one sequence). ``p`` maps parameter names to bf16 tensors."""
     S, d, Hq, Hkv = x.shape[0], cfg.head_dim, cfg.heads, cfg.kv_heads
-    ours = impl == "ours"
-    lin = _Linear.apply if ours else (lambda a, w: F.linear(a, w))
-    norm = (lambda a, g: _RMSNorm.apply(a, g, cfg.eps)) if ours else (lambda a, g: _rms_torch(a, g, cfg.eps))
-    h = norm(x, p["norm1"])
-    qkv = lin(h, p["wqkv"])
-    if ours:
-        q, k, v = _SplitQKV.apply(qkv, Hq, Hkv, d)
-    else:
-        q = qkv[:, :Hq * d].reshape(1, S, Hq, d)
-        k = qkv[:, Hq * d:(Hq + Hkv) * d].reshape(1, S, Hkv, d)
-        v = qkv[:, (Hq + Hkv) * d:].reshape(1, S, Hkv, d).contiguous()
-    scale = 1.0 / math.sqrt(d)
-    if ours:
-        q, k = _Rope.apply(q, cos, sin), _Rope.apply(k, cos, sin)
-        att = _FlashAttention.apply(q, k, v, scale)
-    else:
-        q, k = _rot_half(q, cos, sin), _rot_half(k, cos, sin)
-        att = F.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True,
-                                             scale=scale, enable_gqa=True).transpose(1, 2)
-    x = x + lin(att.reshape(S, Hq * d), p["wo"])
-    h2 = norm(x, p["norm2"])
-    gu = lin(h2, p["wgu"])
-    a = _SwiGLU.apply(gu) if ours else F.silu(gu[:, :cfg.ffn]) * gu[:, cfg.ffn:]
-    return x + lin(a.contiguous(), p["wdown"])
+    qkv = F.linear(_rms_torch(x, p["norm1"], cfg.eps), p["wqkv"])
+    q = qkv[:, :Hq * d].reshape(1, S, Hq, d)
+    k = qkv[:, Hq * d:(Hq + Hkv) * d].reshape(1, S, Hkv, d)
+    v = qkv[:, (Hq + Hkv) * d:].reshape(1, S, Hkv, d).contiguous()
+    q, k = _rot_half(q, cos, sin), _rot_half(k, cos, sin)
+    att = F.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True,
+                                         scale=1.0 / math.sqrt(d), enable_gqa=True).transpose(1, 2)
+    x = x + F.linear(att.reshape(S, Hq * d), p["wo"])
+    gu = F.linear(_rms_torch(x, p["norm2"], cfg.eps), p["wgu"])
+    return x + F.linear((F.silu(gu[:, :cfg.ffn]) * gu[:, cfg.ffn:]).contiguous(), p["wdown"])
 
 
 class _SplitFlat(torch.autograd.Function):
@@ -261,63 +133,41 @@ def split_layer_params(cfg: LlamaConfig, flat: torch.Tensor) -> dict:
 
 
 class _VocabParallelLoss(torch.autograd.Function):
-    """Mean cross-entropy of ``hidden_all @ head_shard.T`` with the vocabulary sharded over the ranks.
-
-    forward : local logits GEMM, one pass of row statistics, ONE packed exchange, loss per token
-    backward: d logits = (softmax - onehot) / tokens from the saved log-sum-exp; d hidden through the
-              MN-major-B GEMM (the caller reduce-scatters it to the token owners); d head = dlogits^T hidden
-    """
+    """Mean cross-entropy of ``hidden_all @ head_shard.T`` with the vocabulary sharded over the ranks, on PyTorch library ops:
+    local logits, one pass of row statistics, ONE packed exchange, loss per token; the backward recomputes the softmax from the
+    saved log-sum-exp."""
 
     @staticmethod
-    def forward(ctx, hidden_all, head_shard, targets_all, comm, vocab_start, impl):
-        ours = impl == "ours"
-        if ours:
-            from ..ops import ce_local_stats, gemm_bf16
-
-            logits = gemm_bf16(hidden_all, head_shard)
-            stats = ce_local_stats(logits, targets_all, vocab_start)
-            allst = comm.all_gather(stats) if comm is not None and comm.size() > 1 else stats.unsqueeze(0)
+    def forward(ctx, hidden_all, head_shard, targets_all, vocab_start):
+        logits = F.linear(hidden_all, head_shard)
+        lf = logits.float()
+        mx = lf.max(-1).values
+        se = torch.exp(lf - mx[:, None]).sum(-1)
+        t = targets_all - vocab_start
+        inr = (t >= 0) & (t < lf.shape[1])
+        tg = torch.where(inr, lf.gather(1, t.clamp(0, lf.shape[1] - 1)[:, None])[:, 0], torch.zeros_like(mx))
+        stats = torch.stack([mx, se, tg], -1)
+        if dist.is_initialized() and dist.get_world_size() > 1:
+            allst = torch.empty((dist.get_world_size(), *stats.shape), device=stats.device)
+            dist.all_gather_into_tensor(allst.view(-1, 3), stats.contiguous())
         else:
-            logits = F.linear(hidden_all, head_shard)
-            lf = logits.float()
-            mx = lf.max(-1).values
-            se = torch.exp(lf - mx[:, None]).sum(-1)
-            t = targets_all - vocab_start
-            inr = (t >= 0) & (t < lf.shape[1])
-            tg = torch.where(inr, lf.gather(1, t.clamp(0, lf.shape[1] - 1)[:, None])[:, 0], torch.zeros_like(mx))
-            stats = torch.stack([mx, se, tg], -1)
-            if dist.is_initialized() and dist.get_world_size() > 1:
-                allst = torch.empty((dist.get_world_size(), *stats.shape), device=stats.device)
-                dist.all_gather_into_tensor(allst.view(-1, 3), stats.contiguous())
-            else:
-                allst = stats.unsqueeze(0)
+            allst = stats.unsqueeze(0)
         gmax = allst[..., 0].max(0).values
         lse = torch.log((allst[..., 1] * torch.exp(allst[..., 0] - gmax)).sum(0)) + gmax
         loss = (lse - allst[..., 2].sum(0)).mean()
         ctx.save_for_backward(hidden_all, head_shard, logits, lse, targets_all)
-        ctx.vocab_start, ctx.ours = vocab_start, ours
+        ctx.vocab_start = vocab_start
         return loss
 
     @staticmethod
     def backward(ctx, dloss):
         hidden_all, head_shard, logits, lse, targets = ctx.saved_tensors
-        n = logits.shape[0]
-        if ctx.ours and logits.dtype == torch.bfloat16 and logits.shape[1] % 8 == 0:
-            from ..ops import ce_backward, gemm_bf16_kn, gemm_bf16_tn
-
-            dlog = ce_backward(logits, lse, targets, ctx.vocab_start, 1.0 / n, upstream=dloss)
-            return gemm_bf16_kn(dlog, head_shard), gemm_bf16_tn(dlog, hidden_all), None, None, None, None
         dlog = torch.exp(logits.float() - lse[:, None])
         t = targets - ctx.vocab_start
-        inr = (t >= 0) & (t < logits.shape[1])
-        rows = torch.nonzero(inr, as_tuple=True)[0]
+        rows = torch.nonzero((t >= 0) & (t < logits.shape[1]), as_tuple=True)[0]
         dlog[rows, t[rows]] -= 1.0
-        dlog = (dlog * (dloss / n)).to(logits.dtype)
-        if ctx.ours:
-            from ..ops import gemm_bf16_kn, gemm_bf16_tn
-
-            return gemm_bf16_kn(dlog, head_shard), gemm_bf16_tn(dlog, hidden_all), None, None, None, None
-        return dlog @ head_shard, dlog.t() @ hidden_all, None, None, None, None
+        dlog = (dlog * (dloss / logits.shape[0])).to(logits.dtype)
+        return dlog @ head_shard, dlog.t() @ hidden_all, None, None
 
 
 # =================================================================================================
@@ -383,11 +233,7 @@ class _Unit:
         if eng.impl == "ours":
             from ..ops import fp8_dequantize_1x128
 
-            if eng.W > 1:
-                q = eng.comm.all_gather(self.q8).view(-1)
-                s = eng.comm.all_gather(self.s8).view(-1)
-            else:
-                q, s = self.q8, self.s8
+            q, s = self.gather_wire()
             return fp8_dequantize_1x128(q.view(-1, 128), s.view(-1, 1), torch.bfloat16).view(-1)
         if eng.W > 1:
             full = torch.empty(self.padded, device=eng.device, dtype=torch.bfloat16)
@@ -395,19 +241,31 @@ class _Unit:
             return full
         return self.bf16.clone()
 
+    def gather_wire(self):
+        """The whole group's parameters in wire format: e4m3 bytes [padded] and fp32 scales [padded / 128]."""
+        eng = self.eng
+        if eng.W > 1:
+            return eng.comm.all_gather(self.q8).view(-1), eng.comm.all_gather(self.s8).view(-1)
+        return self.q8, self.s8
+
+    def reduce_and_step_wire(self, q: torch.Tensor, s: torch.Tensor, step: int) -> None:
+        """``q, s``: the full gradient as e4m3 bytes and 1x128 scales. Exchange, then the fused sum + AdamW + requantise."""
+        from ..ops.quant import fsdp_adamw_fp8
+
+        eng, cfg = self.eng, self.eng.cfg
+        q, s = q.view(eng.W, self.shard), s.view(eng.W, self.shard // 128)
+        if eng.W > 1:
+            q, s = eng.comm.all_to_all(q), eng.comm.all_to_all(s)      # fp8 slices travel, 1 byte/element
+        fsdp_adamw_fp8(q, s, self.master, self.m, self.v, self.q8, self.s8, lr=cfg.lr, beta1=cfg.beta1, beta2=cfg.beta2,
+                       eps=cfg.adam_eps, weight_decay=cfg.weight_decay, grad_scale=1.0, step=step)
+
     def reduce_and_step(self, grad: torch.Tensor, step: int) -> None:
         eng, cfg = self.eng, self.eng.cfg
         if eng.impl == "ours":
             from ..ops import fp8_quantize_1x128
-            from ..ops.quant import fsdp_adamw_fp8
 
             q, s = fp8_quantize_1x128(grad.view(-1, 128))
-            q, s = q.view(eng.W, self.shard), s.view(eng.W, self.shard // 128)
-            if eng.W > 1:
-                q, s = eng.comm.all_to_all(q), eng.comm.all_to_all(s)      # fp8 slices travel, 1 byte/element
-            fsdp_adamw_fp8(q, s, self.master, self.m, self.v, self.q8, self.s8, lr=cfg.lr, beta1=cfg.beta1, beta2=cfg.beta2,
-                           eps=cfg.adam_eps, weight_decay=cfg.weight_decay, grad_scale=1.0, step=step)
-            return
+            return self.reduce_and_step_wire(q, s, step)
         if eng.W > 1:
             gs = torch.empty(self.shard, device=eng.device, dtype=grad.dtype)
             dist.reduce_scatter_tensor(gs, grad.contiguous())
@@ -445,6 +303,7 @@ class FSDPLlama:
         self.final_gain = torch.ones(1, cfg.hidden, device=self.device, dtype=torch.bfloat16)
         self.cos, self.sin = rope_tables(cfg, self.device)
         self.steps = 0
+        self._layer_plan = None
 
     # -- sharded checkpoint --------------------------------------------------------------------------
     def save_sharded(self, directory: str) -> str:
@@ -522,9 +381,77 @@ class FSDPLlama:
 
     # -- one training step -------------------------------------------------------------------------
     def step(self, tokens: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
-        cfg = self.cfg
         self.steps += 1
-        step = self.steps
+        return self._step_ours(tokens, targets) if self.impl == "ours" else self._step_torch(tokens, targets)
+
+    def _layer(self):
+        from ..ops.decoder import DecoderLayer
+
+        cfg = self.cfg
+        if self._layer_plan is None:
+            self._layer_plan = DecoderLayer(cfg.seq, cfg.hidden, cfg.ffn, cfg.heads, cfg.kv_heads, cfg.head_dim, cfg.eps, 1.0 / math.sqrt(cfg.head_dim))
+        return self._layer_plan
+
+    @torch.no_grad()
+    def _step_ours(self, tokens: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+        """Forward and backward in the order the data allows, without a tape: every layer is one native call each way, and a
+        group's gradient is exchanged and applied as soon as it exists."""
+        from ..ops import adam_step, ce_backward, ce_local_stats, gemm_bf16, gemm_bf16_kn, gemm_bf16_tn, rmsnorm, rmsnorm_bwd
+        from ..ops.decoder import ce_loss, embed_fp8, embed_grad_fp8, embed_grad_fp8_supported
+
+        cfg, step, dev = self.cfg, self.steps, self.device
+        if tokens.numel() != cfg.seq:
+            raise ValueError(f"the step takes {cfg.seq} tokens (cfg.seq), got {tokens.numel()}")
+        tok = tokens.reshape(-1).to(torch.int64).contiguous()
+        layer = self._layer()
+        scratch = torch.empty(max(layer.fwd_scratch_bytes, layer.bwd_scratch_bytes), dtype=torch.uint8, device=dev)
+        # ---- forward
+        if cfg.hidden % 16 == 0:
+            x = embed_fp8(*self.embed.gather_wire(), tok, cfg.vocab, cfg.hidden)
+        else:
+            x = F.embedding(tok, self.embed.gather()[:cfg.vocab * cfg.hidden].view(cfg.vocab, cfg.hidden))
+        tape = []
+        for unit in self.units:
+            flat = unit.gather()
+            out, saved = layer.forward(x, flat, self.cos, self.sin, scratch)
+            tape.append((unit, x, flat, saved))
+            x = out
+        xn = rmsnorm(x, self.final_gain.reshape(-1), cfg.eps)
+        hidden_all = self.all_gather_rows(xn)
+        targets_all = self._gather_targets(targets)
+        vocab_start = self.rank * (cfg.vocab // self.W)
+        head = self.head.detach()
+        logits = gemm_bf16(hidden_all, head)
+        stats = ce_local_stats(logits, targets_all, vocab_start)
+        loss, lse = ce_loss(self.comm.all_gather(stats) if self.W > 1 else stats.unsqueeze(0))
+        # ---- backward. Vocabulary-parallel head: every rank saw all tokens, so its gradient is already complete
+        dlog = ce_backward(logits, lse, targets_all, vocab_start, 1.0 / logits.shape[0])
+        del logits
+        dhead = gemm_bf16_tn(dlog, hidden_all)
+        dxn = self.reduce_scatter_rows(gemm_bf16_kn(dlog, head))
+        del dlog
+        adam_step(self.head_master, self.head_m, self.head_v, dhead, lr=cfg.lr, beta1=cfg.beta1, beta2=cfg.beta2, eps=cfg.adam_eps,
+                  step=step, weight_decay=cfg.weight_decay, decoupled=True, p_bf16=self.head.data)
+        del dhead
+        dx, _ = rmsnorm_bwd(x, self.final_gain, dxn, cfg.eps)
+        while tape:
+            unit, x, flat, saved = tape.pop()
+            dflat = torch.empty(unit.padded, dtype=torch.bfloat16, device=dev)
+            if unit.padded > unit.numel:
+                dflat[unit.numel:].zero_()
+            dx = layer.backward(x, flat, self.cos, self.sin, saved, dx, dflat, scratch)
+            del flat, saved, x
+            unit.reduce_and_step(dflat, step)
+            del dflat
+        if embed_grad_fp8_supported(tok.numel(), cfg.hidden):
+            self.embed.reduce_and_step_wire(*embed_grad_fp8(dx, tok, cfg.vocab, cfg.hidden, self.embed.padded), step)
+        else:
+            g = torch.ops.aten.embedding_dense_backward(dx, tok, cfg.vocab, -1, False).reshape(-1)
+            self.embed.reduce_and_step(F.pad(g, (0, self.embed.padded - g.numel())), step)
+        return loss
+
+    def _step_torch(self, tokens: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+        cfg, step = self.cfg, self.steps
 
         def hooked(unit):
             flat = unit.gather().requires_grad_()
@@ -539,28 +466,18 @@ class FSDPLlama:
         x = F.embedding(tokens, emb[:cfg.vocab * cfg.hidden].view(cfg.vocab, cfg.hidden))
         for unit in self.units:
             flat = hooked(unit)
-            x = layer_forward(cfg, split_layer_params(cfg, flat), x, self.cos, self.sin, self.impl)
-        xn = _RMSNorm.apply(x, self.final_gain, cfg.eps) if self.impl == "ours" else _rms_torch(x, self.final_gain, cfg.eps)
-        hidden_all = _GatherRows.apply(xn, self)
-        loss = _VocabParallelLoss.apply(hidden_all, self.head, self._gather_targets(targets), self.comm,
-                                        self.rank * (cfg.vocab // self.W), self.impl)
+            x = layer_forward(cfg, split_layer_params(cfg, flat), x, self.cos, self.sin)
+        hidden_all = _GatherRows.apply(_rms_torch(x, self.final_gain, cfg.eps), self)
+        loss = _VocabParallelLoss.apply(hidden_all, self.head, self._gather_targets(targets), self.rank * (cfg.vocab // self.W))
         loss.backward()
         # vocabulary-parallel head: every rank saw all tokens, so its gradient is already complete
-        g = self.head.grad
-        if self.impl == "ours":
-            from ..ops import adam_step
-
-            with torch.no_grad():
-                adam_step(self.head_master, self.head_m, self.head_v, g.contiguous(), lr=cfg.lr, beta1=cfg.beta1, beta2=cfg.beta2,
-                          eps=cfg.adam_eps, step=step, weight_decay=cfg.weight_decay, decoupled=True, p_bf16=self.head.data)
-        else:
-            with torch.no_grad():
-                gf = g.float()
-                self.head_master.mul_(1.0 - cfg.lr * cfg.weight_decay)
-                self.head_m.mul_(cfg.beta1).add_(gf, alpha=1.0 - cfg.beta1)
-                self.head_v.mul_(cfg.beta2).addcmul_(gf, gf, value=1.0 - cfg.beta2)
-                denom = (self.head_v / (1.0 - cfg.beta2 ** step)).sqrt_().add_(cfg.adam_eps)
-                self.head_master.addcdiv_(self.head_m, denom, value=-cfg.lr / (1.0 - cfg.beta1 ** step))
-                self.head.data.copy_(self.head_master)
+        with torch.no_grad():
+            gf = self.head.grad.float()
+            self.head_master.mul_(1.0 - cfg.lr * cfg.weight_decay)
+            self.head_m.mul_(cfg.beta1).add_(gf, alpha=1.0 - cfg.beta1)
+            self.head_v.mul_(cfg.beta2).addcmul_(gf, gf, value=1.0 - cfg.beta2)
+            denom = (self.head_v / (1.0 - cfg.beta2 ** step)).sqrt_().add_(cfg.adam_eps)
+            self.head_master.addcdiv_(self.head_m, denom, value=-cfg.lr / (1.0 - cfg.beta1 ** step))
+            self.head.data.copy_(self.head_master)
         self.head.grad = None
         return loss.detach()

@@ -82,3 +82,109 @@ def test_adam_vector_and_scalar_forms(n, offset):
     torch.testing.assert_close(v.double(), vd, rtol=1e-5, atol=1e-8)
     torch.testing.assert_close(p.double(), want, rtol=1e-6, atol=1e-6)
     assert torch.equal(pb, p.to(torch.bfloat16))
+
+
+# columns at the edges of the one-, two- and four-chunk forms
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 2048), (5, 2056), (5, 4096), (2, 4104), (1300, 8192)])
+def test_add_rmsnorm_equals_the_separate_passes(rows, cols):
+    import ctypes
+
+    from parallelkernelbench_b200 import _native as nv
+    from parallelkernelbench_b200.ops import rmsnorm
+
+    x, y = (torch.randn(rows, cols, device="cuda", generator=_gen(s)).to(torch.bfloat16) for s in (1, 2))
+    g = torch.randn(cols, device="cuda", generator=_gen(3)).to(torch.bfloat16)
+    total, out = torch.empty_like(x), torch.empty_like(x)
+    nv.check(nv.cuda_lib().pkb_add_rmsnorm_bf16(nv.ptr(x), nv.ptr(y), nv.ptr(g), nv.ptr(total), nv.ptr(out), rows, cols,
+                                                ctypes.c_float(1e-5), nv.current_stream()))
+    assert torch.equal(total, x + y)
+    # the same sum of squares in the same order of threads; the order inside a thread may differ: one ulp of bf16
+    torch.testing.assert_close(out.float(), rmsnorm(x + y, g, 1e-5).float(), rtol=2 ** -7, atol=1e-6)
+
+
+@pytest.mark.parametrize("tokens,hq,hkv,d", [(1, 1, 1, 64), (37, 4, 2, 128), (130, 8, 8, 64)])
+def test_qkv_rope_split_and_merge(tokens, hq, hkv, d):
+    from parallelkernelbench_b200 import _native as nv
+    from parallelkernelbench_b200.ops import rope
+
+    lib, st = nv.cuda_lib(), nv.current_stream()
+    qkv = torch.randn(tokens, (hq + 2 * hkv) * d, device="cuda", generator=_gen(1)).to(torch.bfloat16)
+    ang = torch.rand(tokens, d // 2, device="cuda", generator=_gen(2)) * 6.28
+    cos, sin = torch.cat([ang.cos(), ang.cos()], -1).to(torch.bfloat16), torch.cat([ang.sin(), ang.sin()], -1).to(torch.bfloat16)
+    q = torch.empty(tokens, hq, d, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.empty(tokens, hkv, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    nv.check(lib.pkb_qkv_rope_split(nv.ptr(qkv), nv.ptr(cos), nv.ptr(sin), nv.ptr(q), nv.ptr(k), nv.ptr(v), tokens, hq, hkv, d, st))
+    parts = qkv.view(tokens, hq + 2 * hkv, d)
+    assert torch.equal(q, rope(parts[:, :hq], cos, sin))
+    assert torch.equal(k, rope(parts[:, hq:hq + hkv], cos, sin))
+    assert torch.equal(v, parts[:, hq + hkv:])
+    dq, dk, dv = (torch.randn(tokens, h, d, device="cuda", generator=_gen(h + 5)) for h in (hq, hkv, hkv))
+    got = torch.empty_like(qkv)
+    nv.check(lib.pkb_qkv_rope_merge(nv.ptr(dq), nv.ptr(dk), nv.ptr(dv), nv.ptr(cos), nv.ptr(sin), nv.ptr(got), tokens, hq, hkv, d, st))
+    back = lambda g: rope(g, cos.float(), -sin.float())      # noqa: E731  fp32 rotation, rounded once below
+    want = torch.cat([back(dq), back(dk), dv], 1).reshape(tokens, -1)
+    torch.testing.assert_close(got.float(), want, rtol=2 ** -8, atol=1e-6)
+
+
+# repeated tokens (first, last and middle positions), more positions than one mask word, the two ends of the table
+@pytest.mark.parametrize("n,vocab,H", [(1, 5, 128), (33, 7, 256), (257, 1000, 640)])
+def test_embedding_wire_format(n, vocab, H):
+    from parallelkernelbench_b200.ops import fp8_dequantize_1x128, fp8_quantize_1x128
+    from parallelkernelbench_b200.ops.decoder import embed_fp8, embed_grad_fp8
+
+    table = torch.randn(vocab, H, device="cuda", generator=_gen(1))
+    q, s = fp8_quantize_1x128(table)
+    tok = torch.randint(0, vocab, (n,), device="cuda", generator=_gen(2))
+    tok[0], tok[-1] = vocab - 1, vocab - 1 if n > 1 else vocab - 1
+    x = embed_fp8(q.view(-1), s.view(-1), tok, vocab, H)
+    assert torch.equal(x, fp8_dequantize_1x128(q, s)[tok])
+    dx = torch.randn(n, H, device="cuda", generator=_gen(3)).to(torch.bfloat16)
+    padded = vocab * H + 256
+    gq, gs = embed_grad_fp8(dx, tok, vocab, H, padded)
+    dense = torch.zeros(vocab, H, device="cuda")
+    for i in range(n):                                    # fp32 sums in position order
+        dense[tok[i]] += dx[i].float()
+    wq, ws = fp8_quantize_1x128(torch.nn.functional.pad(dense.to(torch.bfloat16).reshape(-1), (0, 256)).view(-1, 128))
+    assert torch.equal(gq, wq.view(-1)) and torch.equal(gs, ws.view(-1))
+
+
+@pytest.mark.parametrize("rows,W", [(1, 1), (1025, 3)])
+def test_ce_loss_of_several_shards(rows, W):
+    from parallelkernelbench_b200.ops.decoder import ce_loss
+
+    lg = torch.randn(W, rows, 50, device="cuda", generator=_gen(1)) * 5
+    mx = lg.max(-1).values
+    st = torch.stack([mx, torch.exp(lg - mx[..., None]).sum(-1), torch.zeros_like(mx)], -1)
+    st[0, :, 2] = lg[0, :, 7]
+    loss, lse = ce_loss(st.contiguous())
+    ref = torch.logsumexp(lg.double().permute(1, 0, 2).reshape(rows, -1), -1)
+    torch.testing.assert_close(lse.double(), ref, rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(loss.double(), (ref - lg[0, :, 7].double()).mean(), rtol=1e-5, atol=1e-5)
+
+
+# below and above the row count at which the forward GEMMs change form; a ragged number of tokens; both head dimensions
+@pytest.mark.parametrize("S,H,Fn,hq,hkv,d", [(65, 256, 384, 4, 2, 64), (700, 512, 640, 4, 4, 128)])
+def test_decoder_layer_against_autograd(S, H, Fn, hq, hkv, d):
+    from parallelkernelbench_b200.models.llama import LlamaConfig, layer_forward, rope_tables, split_layer_params
+    from parallelkernelbench_b200.ops.decoder import DecoderLayer
+
+    cfg = LlamaConfig(layers=1, hidden=H, ffn=Fn, heads=hq, kv_heads=hkv, vocab=64, seq=S)
+    assert cfg.head_dim == d
+    flat = torch.randn(cfg.layer_numel(), device="cuda", generator=_gen(1)) * 0.05
+    flat[-2 * H:] = 1 + 0.1 * flat[-2 * H:]
+    flat = flat.to(torch.bfloat16)
+    x, dout = (torch.randn(S, H, device="cuda", generator=_gen(s)).to(torch.bfloat16) for s in (2, 3))
+    cos, sin = rope_tables(cfg, "cuda")
+    L = DecoderLayer(S, H, Fn, hq, hkv, d, cfg.eps, d ** -0.5)
+    scratch = torch.empty(max(L.fwd_scratch_bytes, L.bwd_scratch_bytes), dtype=torch.uint8, device="cuda")
+    out, saved = L.forward(x, flat, cos, sin, scratch)
+    dflat = torch.full_like(flat, float("nan"))
+    dx = L.backward(x, flat, cos, sin, saved, dout, dflat, scratch)
+    xr, fr = x.double().requires_grad_(), flat.double().requires_grad_()
+    with torch.nn.attention.sdpa_kernel(torch.nn.attention.SDPBackend.MATH):
+        ref = layer_forward(cfg, split_layer_params(cfg, fr), xr, cos.double(), sin.double())
+        ref.backward(dout.double())
+    # every intermediate tensor is rounded to bf16 (2^-9 each); a dozen of them lie between input and result
+    for got, want in ((out, ref.detach()), (dx, xr.grad), (dflat, fr.grad)):
+        assert torch.isfinite(got).all()
+        assert float((got.double() - want).norm() / want.norm()) < 1.5e-2

@@ -12,12 +12,11 @@
 
 #include "pkb/api.h"
 #include "pkb/collectives_api.h"
+#include "pkb/fp8_block.cuh"
 #include "pkb/host.h"
 #include "pkb/symm.cuh"
 
 namespace pkb {
-
-constexpr float kInv448 = 1.0f / 448.0f;
 
 // ================================================================================================
 // RoPE (rotate-half): x is [tokens, heads, dim]; cos/sin are [tokens, dim] (the two halves of a row
@@ -87,20 +86,10 @@ __global__ void __launch_bounds__(256) fp8_quant_kernel(const T* __restrict__ x,
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
     if (t >= nthr) continue;
-    float s = amax * kInv448;   // amax / 448 the way PyTorch evaluates a tensor divided by a Python scalar on the GPU: times the rounded reciprocal
-    if (pow2_scales && s > 0.f) s = exp2f(ceilf(log2f(s)));  // power-of-two scale (exact to undo)
-    if (s == 0.f) s = 1.0f;
-    // the correctly rounded quotient x / s, not x * (1 / s): the quotient decides the e4m3 code at rounding boundaries, and
-    // x / s is what the PyTorch formulation computes. One reciprocal per block, then per element a product, its residual
-    // and one correction (three FMA-pipe instructions instead of a division each).
-    const float inv = __frcp_rn(s);
+    const float s = fp8_block_scale(amax, pow2_scales);
     uint32_t o[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(div_rn_by(v[4 * j], s, inv), div_rn_by(v[4 * j + 1], s, inv)), __NV_SATFINITE, __NV_E4M3);
-      const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(div_rn_by(v[4 * j + 2], s, inv), div_rn_by(v[4 * j + 3], s, inv)), __NV_SATFINITE, __NV_E4M3);
-      o[j] = (uint32_t)lo | ((uint32_t)hi << 16);
-    }
+    fp8_encode8(v, s, o);
+    fp8_encode8(v + 8, s, o + 2);
     st_global_v4(y + (t << 4), U4{o[0], o[1], o[2], o[3]});
     if ((t & 7) == 0) scales[t >> 3] = s;
   }
@@ -124,14 +113,8 @@ __global__ void __launch_bounds__(256) fp8_dequant_kernel(const uint8_t* __restr
     const float sc = scales[t >> 3];
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
     float v[16];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      __half2_raw h0 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[j] & 0xffffu), __NV_E4M3);
-      __half2_raw h1 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[j] >> 16), __NV_E4M3);
-      const float2 f0 = __half22float2(*reinterpret_cast<__half2*>(&h0));
-      const float2 f1 = __half22float2(*reinterpret_cast<__half2*>(&h1));
-      v[4 * j] = f0.x * sc; v[4 * j + 1] = f0.y * sc; v[4 * j + 2] = f1.x * sc; v[4 * j + 3] = f1.y * sc;
-    }
+    fp8_decode8(w, sc, v);
+    fp8_decode8(w + 2, sc, v + 8);
     T* o = x + (t << 4);
     if constexpr (sizeof(T) == 2) {
       st_global_v4(o, U4{pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7])});

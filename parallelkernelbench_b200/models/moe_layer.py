@@ -68,8 +68,11 @@ class EPMoELayer:
         else:
             self.h = torch.empty((self.ex.capacity, cfg.inter), dtype=torch.bfloat16, device=dev)
 
+    def _logits(self, x: torch.Tensor) -> torch.Tensor:
+        return gemm_bf16(x, self.w_router, out_dtype=torch.float32, mode="single", block_n=128)
+
     def route(self, x: torch.Tensor):
-        logits = gemm_bf16(x, self.w_router, out_dtype=torch.float32, mode="single", block_n=128)
+        logits = self._logits(x)
         if self.cfg.fused_router:
             gates, idx, _ = route_topk(logits, self.router_bias_f32, self.cfg.top_k, counts=self.ex.counts)
             return gates, idx
@@ -80,9 +83,13 @@ class EPMoELayer:
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         T = x.shape[0]
-        gates, idx = self.route(x)
-        flat_idx = idx.view(-1)
-        self.ex.plan(flat_idx, self.comm, counts_ready=self.cfg.fused_router)
+        if self.cfg.fused_router:
+            gates, idx = self.ex.route(self._logits(x), self.router_bias_f32, self.comm)
+            flat_idx = idx.view(-1)
+        else:
+            gates, idx = self.route(x)
+            flat_idx = idx.view(-1)
+            self.ex.plan(flat_idx, self.comm)
         if self.cfg.fp8_experts:
             x8, xs = self.ex.dispatch(x, flat_idx, dequantize=False)
             gemm_fp8_blockscaled(x8, xs, self.w8_gate_up, self.s_gate_up, offsets=self.ex.offsets, epilogue="swiglu_quant",

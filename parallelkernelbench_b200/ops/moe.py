@@ -123,7 +123,31 @@ class MoEExchange:
         self.cursor = torch.zeros(num_experts, dtype=torch.int32, device=dev)
         self.offsets = torch.zeros(self.El + 1, dtype=torch.int32, device=dev)
         self.overflow = torch.zeros(1, dtype=torch.int32, device=dev)
+        self.route_work = torch.zeros(num_experts + 1, dtype=torch.int32, device=dev)   # zero between calls
         self.slots = None
+
+    # -- routing -------------------------------------------------------------------------------
+    def route(self, logits: torch.Tensor, bias: torch.Tensor | None, comm):
+        """:func:`route_topk` into this exchange's ``counts``, followed by :meth:`plan`. For a group of one rank both are one
+        launch. Returns ``(gates [T, k], idx [T, k])``."""
+        if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1 or logits.shape[1] != self.E:
+            raise TypeError("logits must be fp32 [T, E] with unit inner stride")
+        if self.E > 256:
+            raise ValueError("at most 256 experts")
+        if bias is not None and (bias.dtype != torch.float32 or bias.numel() != self.E or not bias.is_contiguous()):
+            raise TypeError("bias must be contiguous fp32 [E]")
+        T = logits.shape[0]
+        gates = torch.empty((T, self.top_k), dtype=torch.float32, device=logits.device)
+        idx = torch.empty((T, self.top_k), dtype=torch.int32, device=logits.device)
+        alone = self.group.size == 1
+        plan = (self.seg_base, self.offsets, self.cursor) if alone else (None, None, None)
+        nv.check(nv.cuda_lib().pkb_moe_route_plan(nv.ptr(logits), nv.c_ll(logits.stride(0)), nv.ptr(bias), T, self.E, self.top_k,
+                                                  nv.ptr(gates), nv.ptr(idx), nv.ptr(self.counts), nv.ptr(self.route_work),
+                                                  *map(nv.ptr, plan), nv.current_stream()), "pkb_moe_route_plan")
+        nv.count_launch()
+        if not alone:
+            self.plan(idx.view(-1), comm, counts_ready=True)
+        return gates, idx
 
     # -- planning ------------------------------------------------------------------------------
     def plan(self, expert_idx: torch.Tensor, comm, counts_ready: bool = False) -> torch.Tensor:
@@ -147,37 +171,64 @@ class MoEExchange:
         ``[capacity, hidden]`` (rows ``[0, offsets[-1])`` are valid, expert-major); with
         ``dequantize=False`` (fp8 dispatch only) the received e4m3 bytes ``[capacity, hidden]`` and their fp32
         scales ``[capacity, >= hidden/128]`` instead, as views of the receive buffers."""
-        from .elementwise import fp8_dequantize_1x128, fp8_quantize_1x128
-
         T = x.shape[0]
-        self.slots = torch.empty(T * self.top_k, dtype=torch.int32, device=x.device)
-        if self.fp8:
-            payload, scales = fp8_quantize_1x128(x)
-            if self.scale_bytes != scales.shape[1] * 4:
-                pad = torch.zeros((T, self.scale_bytes // 4), dtype=torch.float32, device=x.device)
-                pad[:, :scales.shape[1]] = scales
-                scales = pad
-        else:
-            payload, scales = x.contiguous(), None
-        nv.check(nv.cuda_lib().pkb_moe_dispatch_meta(
-            self.group.ref, nv.ptr(payload), nv.ptr(scales), self.payload_bytes, self.scale_bytes, nv.ptr(expert_idx),
-            nv.c_ll(T * self.top_k), self.top_k, self.El, nv.ptr(self.seg_base), nv.ptr(self.cursor), nv.ptr(self.slots),
-            ctypes.c_ulonglong(self.recv_payload.offset), ctypes.c_ulonglong(self.recv_scales.offset), self.capacity,
-            nv.ptr(self.overflow), ctypes.c_ulonglong(self.recv_meta.offset if self.push_combine else 0),
-            nv.current_stream()), "pkb_moe_dispatch_meta")
-        nv.count_launch()
-        if self.fp8 and not dequantize:
-            return self.recv_payload.local, self.recv_scales.local.view(torch.float32)
-        if not dequantize:
+        lib = nv.cuda_lib()
+        if not self.fp8 and not dequantize:
             raise ValueError("dequantize=False needs the fp8 dispatch")
-        if self.fp8:
-            nblk = self.hidden // 128
-            s = self.recv_scales.local.view(torch.float32)[:, :nblk]
-            if s.shape[1] * 4 != self.scale_bytes:
-                s = s.contiguous()
+        if x.numel() != T * self.hidden:
+            raise ValueError(f"expected tokens of {self.hidden} elements")
+        self.slots = torch.empty(T * self.top_k, dtype=torch.int32, device=x.device)
+        meta_off = ctypes.c_ulonglong(self.recv_meta.offset if self.push_combine else 0)
+        if not self.fp8 or x.dtype != torch.bfloat16:
+            # rows that travel as they are: bf16, or (from fp32 tokens) quantised by a pass of their own
+            payload, scales = (self._quantised(x) if self.fp8 else (x.contiguous(), None))
+            nv.check(lib.pkb_moe_dispatch_meta(
+                self.group.ref, nv.ptr(payload), nv.ptr(scales), self.payload_bytes, self.scale_bytes, nv.ptr(expert_idx),
+                nv.c_ll(T * self.top_k), self.top_k, self.El, nv.ptr(self.seg_base), nv.ptr(self.cursor), nv.ptr(self.slots),
+                ctypes.c_ulonglong(self.recv_payload.offset), ctypes.c_ulonglong(self.recv_scales.offset), self.capacity,
+                nv.ptr(self.overflow), meta_off, nv.current_stream()), "pkb_moe_dispatch_meta")
+            nv.count_launch()
+            if not self.fp8:
+                return self.recv_payload.local.view(torch.bfloat16)
+            recv_scales = self.recv_scales.local.view(torch.float32)
+            if not dequantize:
+                return self.recv_payload.local, recv_scales
+            from .elementwise import fp8_dequantize_1x128
+
             # only the rows that arrived (offsets[-1], on the device) are converted: the buffer has capacity_factor x the mean
-            return fp8_dequantize_1x128(self.recv_payload.local, s, torch.bfloat16, valid_rows=self.offsets[self.El:self.El + 1])
-        return self.recv_payload.local.view(torch.bfloat16)
+            return fp8_dequantize_1x128(self.recv_payload.local, recv_scales[:, :self.hidden // 128], torch.bfloat16,
+                                        valid_rows=self.offsets[self.El:self.El + 1])
+        # bf16 rows are quantised by the dispatch itself; with `dequantize` it writes the rows that stay on this rank as bf16 at
+        # once, and what other ranks sent is converted after its barrier
+        xc = x.contiguous()
+        rows = torch.empty((self.capacity, self.hidden), dtype=torch.bfloat16, device=x.device) if dequantize else None
+        nv.check(lib.pkb_moe_dispatch_quant(
+            self.group.ref, nv.ptr(xc), self.hidden, self.scale_bytes, nv.ptr(expert_idx), nv.c_ll(T * self.top_k), self.top_k,
+            self.El, nv.ptr(self.seg_base), nv.ptr(self.cursor), nv.ptr(self.slots), ctypes.c_ulonglong(self.recv_payload.offset),
+            ctypes.c_ulonglong(self.recv_scales.offset), self.capacity, nv.ptr(self.overflow), meta_off, nv.ptr(rows),
+            nv.current_stream()), "pkb_moe_dispatch_quant")
+        nv.count_launch()
+        if rows is None:
+            return self.recv_payload.local, self.recv_scales.local.view(torch.float32)
+        if self.group.size > 1:
+            first = self.group.rank_in_group * self.El
+            nv.check(lib.pkb_moe_dequant(nv.ptr(self.recv_payload.local), nv.ptr(self.recv_scales.local), self.hidden,
+                                         self.scale_bytes, nv.ptr(self.offsets), nv.ptr(self.seg_base[first:]),
+                                         nv.ptr(self.counts[first:]), self.El, self.capacity, nv.ptr(rows),
+                                         nv.current_stream()), "pkb_moe_dequant")
+            nv.count_launch()
+        return rows
+
+    def _quantised(self, x: torch.Tensor):
+        """e4m3 rows and their scales, padded to the row pitch of the receive buffer."""
+        from .elementwise import fp8_quantize_1x128
+
+        payload, scales = fp8_quantize_1x128(x)
+        if self.scale_bytes != scales.shape[1] * 4:
+            pad = torch.zeros((x.shape[0], self.scale_bytes // 4), dtype=torch.float32, device=x.device)
+            pad[:, :scales.shape[1]] = scales
+            scales = pad
+        return payload, scales
 
     def home_ptrs(self) -> list[int]:
         """Addresses of every member's ``home`` buffer, in group order (what ``recv_meta[:, 0]`` indexes)."""

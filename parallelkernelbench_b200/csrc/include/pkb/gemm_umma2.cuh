@@ -17,6 +17,18 @@ constexpr int kGemm2Stages = 6;
 constexpr int kGemm2ABytes = 128 * kGemmBlockK * 2;   // this CTA's half of A
 constexpr int kGemm2BBytes = 128 * kGemmBlockK * 2;   // this CTA's half of B
 constexpr int kGemm2StageBytes = kGemm2ABytes + kGemm2BBytes;
+// Narrower tiles (BN = 192 or 128: each CTA loads BN / 2 rows of B) for problems whose 256-wide tiles leave the last wave of
+// pairs nearly empty: see pair_tile_n in kernels/gemm.cu for the rule and its figures.
+template <int BN, bool B_MN>
+struct Gemm2Tile {
+  static_assert(BN == 256 || BN == 192 || BN == 128, "tile widths of the CTA-pair kernel");
+  static constexpr int kStages = BN == 128 ? 8 : kGemm2Stages;
+  // an MN-major B comes in 64-column boxes: at BN = 192 half of the second box is not used
+  static constexpr int kBoxesMn = (BN / 2 + 63) / 64;
+  static constexpr int kBBytes = B_MN ? kBoxesMn * 8192 : BN / 2 * kGemmBlockK * 2;
+  static constexpr int kStageBytes = kGemm2ABytes + kBBytes;
+  static_assert(kStages * kStageBytes <= kGemm2Stages * kGemm2StageBytes, "the ring outgrew the shared-memory plan");
+};
 constexpr int kGemm2StoreBytes = 4 * 2 * 4096;      // per epilogue warp: two 32 x 128-byte buffers
 constexpr int kGemm2SmemTotal = kGemm2Stages * kGemm2StageBytes + kGemm2StoreBytes + 256 + 1024;
 
@@ -35,7 +47,7 @@ struct alignas(64) GemmOutMaps {
 // (one weight matrix per group, e.g. the experts of a MoE layer): tiles are (group, 256-row block of the group, n block), rows
 // of a tile beyond the group's end are computed and not stored. Register epilogue only.
 template <int EPI, bool OUT_F32, bool A_READY, bool RS_SCATTER, bool TMA_STORE = false, bool BCAST = false, bool A_MN = false,
-          bool B_MN = false, bool GROUPED = false>
+          bool B_MN = false, bool GROUPED = false, int BN = kGemm2TileN>
 __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b,
                                                const GemmParams& p, const int pair,
                                                const int num_pairs,
@@ -45,21 +57,22 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
   static_assert(!BCAST || (TMA_STORE && !RS_SCATTER), "the broadcast epilogue is a TMA-store epilogue");
   static_assert(!(A_MN && A_READY), "the gathered-A hook loads A K-major");
   static_assert(!GROUPED || (!TMA_STORE && !RS_SCATTER && !A_READY && !A_MN && !B_MN && !OUT_F32), "the grouped form is K-major, bf16, register epilogue");
-  constexpr int kStages = kGemm2Stages;
-  constexpr int BN = kGemm2TileN;
+  using T = Gemm2Tile<BN, B_MN>;
+  constexpr int kStages = T::kStages;
+  constexpr int kAccStride = 256;   // accumulator buffers at columns 0 and 256 for every tile width
   constexpr uint32_t kTmemCols = 512;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t store_base = smem_base + kStages * kGemm2StageBytes;
+  const uint32_t store_base = smem_base + kStages * T::kStageBytes;
   const uint32_t bar_base = store_base + kGemm2StoreBytes;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * kStages + a); };
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * kStages + 2 + a); };
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(
-      smem_gen + kStages * kGemm2StageBytes + kGemm2StoreBytes + 8 * (2 * kStages + 4));
+      smem_gen + kStages * T::kStageBytes + kGemm2StoreBytes + 8 * (2 * kStages + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -149,7 +162,7 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
         if constexpr (GROUPED) tile_rows(tile, g_row0, g_row_end, g_b_row0, n_blk);
         else tile_coords(tile, m_blk, n_blk);
         const int row0 = (GROUPED ? g_row0 : m_blk * kGemm2TileM) + (int)cta_rank * 128;
-        const int col0 = (GROUPED ? g_b_row0 : n_blk * BN) + (int)cta_rank * 128;   // this CTA's 128 rows of B
+        const int col0 = (GROUPED ? g_b_row0 : n_blk * BN) + (int)cta_rank * (BN / 2);   // this CTA's half of the B rows
         const CUtensorMap* map_a = &tmap_a;
         int a_row = row0;
         bool a_is_local = false;
@@ -182,8 +195,8 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
             ok = false;
             break;
           }
-          mbar_expect_tx_p(full_bar(stage), 2 * kGemm2StageBytes, leader ? lead : 0u);
-          const uint32_t sa = smem_base + stage * kGemm2StageBytes;
+          mbar_expect_tx_p(full_bar(stage), 2 * T::kStageBytes, leader ? lead : 0u);
+          const uint32_t sa = smem_base + stage * T::kStageBytes;
           if constexpr (A_MN) {
             tma_load_2d_pair_p(sa, map_a, full_bar(stage), a_row, kb * kGemmBlockK, lead);
             tma_load_2d_pair_p(sa + 8192, map_a, full_bar(stage), a_row + 64, kb * kGemmBlockK, lead);
@@ -192,7 +205,8 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
           }
           if constexpr (B_MN) {
             tma_load_2d_pair_p(sa + kGemm2ABytes, &tmap_b, full_bar(stage), col0, kb * kGemmBlockK, lead);
-            tma_load_2d_pair_p(sa + kGemm2ABytes + 8192, &tmap_b, full_bar(stage), col0 + 64, kb * kGemmBlockK, lead);
+            if constexpr (T::kBoxesMn == 2)
+              tma_load_2d_pair_p(sa + kGemm2ABytes + 8192, &tmap_b, full_bar(stage), col0 + 64, kb * kGemmBlockK, lead);
           } else {
             tma_load_2d_pair_p(sa + kGemm2ABytes, &tmap_b, full_bar(stage), kb * kGemmBlockK, col0, lead);
           }
@@ -215,7 +229,7 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
     if (leader) {
       const uint32_t lead = elect_one() ? 1u : 0u;
       constexpr uint32_t idesc = make_idesc(kGemm2TileM, BN, 1, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      // low descriptor words of stage 0; a stage adds kGemm2StageBytes >> 4, a K step of 16 adds 2 (K-major) or 128 (MN-major)
+      // low descriptor words of stage 0; a stage adds T::kStageBytes >> 4, a K step of 16 adds 2 (K-major) or 128 (MN-major)
       const uint32_t a_lo0 = A_MN ? smem_desc_lo_mnmajor(smem_base, 8192u) : smem_desc_lo_kmajor(smem_base);
       const uint32_t b_lo0 = B_MN ? smem_desc_lo_mnmajor(smem_base + kGemm2ABytes, 8192u) : smem_desc_lo_kmajor(smem_base + kGemm2ABytes);
       int stage = 0;
@@ -229,7 +243,7 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
           break;
         }
         tc_fence_after_sync();
-        const uint32_t tmem_d = tmem_base + acc * BN;
+        const uint32_t tmem_d = tmem_base + acc * kAccStride;
         for (int kb = 0; kb < num_k; ++kb) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag, p.wait_budget_ns)) {
             if (lane == 0) record_status(p.status, kStatusMbarTimeout, p.kernel_id, p.rank, stage, 21, tile);
@@ -237,7 +251,7 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
             break;
           }
           tc_fence_after_sync();
-          const uint32_t a_lo = a_lo0 + stage * (kGemm2StageBytes >> 4), b_lo = b_lo0 + stage * (kGemm2StageBytes >> 4);
+          const uint32_t a_lo = a_lo0 + stage * (T::kStageBytes >> 4), b_lo = b_lo0 + stage * (T::kStageBytes >> 4);
 #pragma unroll
           for (int k = 0; k < kGemmBlockK / 16; ++k)
             umma_f16_ss_pair_p(tmem_d, smem_desc_join(a_lo + (A_MN ? 128u : 2u) * k), smem_desc_join(b_lo + (B_MN ? 128u : 2u) * k), idesc,
@@ -264,6 +278,7 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
     uint32_t acc_phase = 0;
     const uint32_t leader_tempty0 = mapa_shared(tempty_bar(0), 0);
     const uint32_t leader_tempty1 = mapa_shared(tempty_bar(1), 0);
+    [[maybe_unused]] uint32_t store_buf = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int m_blk = 0, n_blk = 0, g_row0 = 0, g_row_end = 0, g_b_row0 = 0;
       if constexpr (GROUPED) tile_rows(tile, g_row0, g_row_end, g_b_row0, n_blk);
@@ -302,12 +317,13 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
         }
 #pragma unroll 1
         for (int c = 0; c < BN / 64; ++c) {
-          const uint32_t buf = stg + static_cast<uint32_t>(c & 1) * 4096u;
+          const uint32_t buf = stg + store_buf;      // the two buffers alternate over tiles as well (BN / 64 may be odd)
+          store_buf ^= 4096u;
           if (lane == 0) tma_store_wait_read<1>();  // the store that last used this buffer was read
           __syncwarp();
           uint32_t r0[32], r1[32];
           const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                                 static_cast<uint32_t>(acc * BN + c * 64);
+                                 static_cast<uint32_t>(acc * kAccStride + c * 64);
           tmem_ld_32x32(taddr, r0);
           tmem_ld_32x32(taddr + 32, r1);
           tmem_ld_wait();
@@ -354,8 +370,8 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
             } else {
               tma_store_2d(&out_maps->m[map_idx], buf, col0, row_coord);
             }
-            tma_store_commit();
           }
+          if (lane == 0) tma_store_commit();   // a group per buffer use, empty where nothing is stored: the wait above counts groups
         }
         if constexpr (RS_SCATTER) {
           // the owner may only be told once the stores have been performed, not merely read
@@ -370,7 +386,7 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
         for (int c = 0; c < BN / 32; ++c) {
           uint32_t r[32];
           const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                                 static_cast<uint32_t>(acc * BN + c * 32);
+                                 static_cast<uint32_t>(acc * kAccStride + c * 32);
           tmem_ld_32x32(taddr, r);
           tmem_ld_wait();
           const int col0 = n0 + c * 32;
@@ -474,20 +490,17 @@ __device__ __forceinline__ void gemm_umma2_cta(const CUtensorMap& tmap_a, const 
   }
 }
 
-template <int EPI, bool OUT_F32, bool A_READY, bool RS_SCATTER>
+template <int EPI, bool OUT_F32, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-gemm_umma2_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                  const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
-  gemm_umma2_cta<EPI, OUT_F32, A_READY, RS_SCATTER>(tmap_a, tmap_b, p, blockIdx.x >> 1,
-                                                    gridDim.x >> 1);
+gemm_umma2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+  gemm_umma2_cta<EPI, OUT_F32, false, false, false, false, false, false, false, BN>(tmap_a, tmap_b, p, blockIdx.x >> 1, gridDim.x >> 1);
 }
 
-// MN-major operands (see gemm_umma2_cta), register epilogue (bf16 or fp32 output)
-template <int EPI, bool OUT_F32, bool A_MN, bool B_MN>
+// MN-major operands (see gemm_umma2_cta), register epilogue (fp32 output, or bf16 rows that a TMA store cannot address)
+template <int EPI, bool OUT_F32, bool A_MN, bool B_MN, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-gemm_umma2_mn_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                     const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
-  gemm_umma2_cta<EPI, OUT_F32, false, false, false, false, A_MN, B_MN>(tmap_a, tmap_b, p, blockIdx.x >> 1, gridDim.x >> 1);
+gemm_umma2_mn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+  gemm_umma2_cta<EPI, OUT_F32, false, false, false, false, A_MN, B_MN, false, BN>(tmap_a, tmap_b, p, blockIdx.x >> 1, gridDim.x >> 1);
 }
 
 // grouped form (see gemm_umma2_cta): one weight matrix per row group, register epilogue
@@ -498,13 +511,12 @@ gemm_umma2_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 }
 
 // bf16 output through the TMA-store epilogue
-template <int EPI>
+template <int EPI, bool A_MN, bool B_MN, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-gemm_umma2_tma_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                      const __grid_constant__ CUtensorMap tmap_b,
+gemm_umma2_tma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const __grid_constant__ GemmOutMaps out_maps, const GemmParams p) {
-  gemm_umma2_cta<EPI, false, false, false, true>(tmap_a, tmap_b, p, blockIdx.x >> 1,
-                                                 gridDim.x >> 1, &out_maps);
+  gemm_umma2_cta<EPI, false, false, false, true, false, A_MN, B_MN, false, BN>(tmap_a, tmap_b, p, blockIdx.x >> 1, gridDim.x >> 1,
+                                                                               &out_maps);
 }
 
 }  // namespace pkb

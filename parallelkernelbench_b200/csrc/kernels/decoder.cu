@@ -15,8 +15,8 @@
 using namespace pkb;
 
 extern "C" {
-int pkb_gemm_bf16_pair(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N, int K,
-                       const void* bias, float alpha, int epilogue, int out_f32, int num_ctas, void* stream);
+int pkb_gemm_bf16_auto(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N, int K,
+                       const void* bias, float alpha, int epilogue, int out_f32, void* stream);
 int pkb_gemm_bf16_bkn(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N, int K,
                       float alpha, int epilogue, int out_f32, void* stream);
 int pkb_gemm_bf16_tn(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N, int K,
@@ -116,8 +116,7 @@ inline void* at(void* base, long long elem) { return static_cast<uint8_t*>(base)
 
 // y[M, N] = x[M, K] w[N, K]^T
 int linear(const void* x, const void* w, void* y, int M, int N, int K, void* stream) {
-  if (M >= 512 && N >= 256) return pkb_gemm_bf16_pair(x, K, w, K, y, N, M, N, K, nullptr, 1.0f, 0, 0, 0, stream);
-  return pkb_gemm_bf16(x, K, w, K, y, N, M, N, K, nullptr, 1.0f, 0, 0, 0, 0, stream);
+  return pkb_gemm_bf16_auto(x, K, w, K, y, N, M, N, K, nullptr, 1.0f, 0, 0, stream);
 }
 // dx[M, K] = dy[M, N] w[N, K]
 int linear_dx(const void* dy, const void* w, void* dx, int M, int N, int K, void* stream) {

@@ -2,6 +2,7 @@
 #include <cstdlib>
 
 #include "pkb/api.h"
+#include "pkb/gemm_split.cuh"
 #include "pkb/gemm_umma2.cuh"
 #include "pkb/host.h"
 
@@ -35,71 +36,142 @@ static int dispatch_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tb, c
   return kApiBadArgument;
 }
 
-template <int EPI, bool OUT_F32>
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                       int num_ctas, cudaStream_t stream) {
-  auto kern = gemm_umma2_kernel<EPI, OUT_F32, false, false>;
-  PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      kGemm2SmemTotal));
-  kern<<<num_ctas, kGemmThreads, kGemm2SmemTotal, stream>>>(ta, tb, p);
-  PKB_CHECK_CUDA(cudaGetLastError());
-  return kApiOk;
-}
-
-template <int EPI>
-static int launch_pair_tma(const CUtensorMap& ta, const CUtensorMap& tb, const GemmOutMaps& om,
-                           const GemmParams& p, int num_ctas, cudaStream_t stream) {
-  auto kern = gemm_umma2_tma_kernel<EPI>;
-  PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      kGemm2SmemTotal));
-  kern<<<num_ctas, kGemmThreads, kGemm2SmemTotal, stream>>>(ta, tb, om, p);
-  PKB_CHECK_CUDA(cudaGetLastError());
-  return kApiOk;
-}
-
-static int dispatch_pair_tma(int epi, const CUtensorMap& ta, const CUtensorMap& tb,
-                             const GemmOutMaps& om, const GemmParams& p, int num_ctas,
-                             cudaStream_t stream) {
-  switch (epi) {
-    case kEpiNone: return launch_pair_tma<kEpiNone>(ta, tb, om, p, num_ctas, stream);
-    case kEpiSilu: return launch_pair_tma<kEpiSilu>(ta, tb, om, p, num_ctas, stream);
-    case kEpiBias: return launch_pair_tma<kEpiBias>(ta, tb, om, p, num_ctas, stream);
-    case kEpiBiasSilu: return launch_pair_tma<kEpiBiasSilu>(ta, tb, om, p, num_ctas, stream);
-  }
-  set_last_error("unknown epilogue");
-  return kApiBadArgument;
-}
-
-template <bool OUT_F32>
-static int dispatch_pair(int epi, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                         int num_ctas, cudaStream_t stream) {
-  switch (epi) {
-    case kEpiNone: return launch_pair<kEpiNone, OUT_F32>(ta, tb, p, num_ctas, stream);
-    case kEpiSilu: return launch_pair<kEpiSilu, OUT_F32>(ta, tb, p, num_ctas, stream);
-    case kEpiBias: return launch_pair<kEpiBias, OUT_F32>(ta, tb, p, num_ctas, stream);
-    case kEpiBiasSilu: return launch_pair<kEpiBiasSilu, OUT_F32>(ta, tb, p, num_ctas, stream);
-  }
-  set_last_error("unknown epilogue");
-  return kApiBadArgument;
-}
-
 // The backward layouts on CTA pairs: PKB_GEMM_PAIR_MN=0 keeps the one-CTA-per-tile kernels.
 static bool pair_mn_enabled() {
   static const bool on = [] { const char* e = getenv("PKB_GEMM_PAIR_MN"); return !(e != nullptr && e[0] == '0'); }();
   return on;
 }
 
+// Tile width of the CTA-pair kernel. A wave is sm_count / 2 tiles of 256 x BN, so a problem costs its number of waves times the
+// width, times a factor for narrow tiles, which read more operand bytes per flop. The factors are measured (us at 256 / 192 /
+// 128): 1333 x 4104 x 4096 (2, 2, 3 waves) 51.9 / 43.8 / 46.0; 4096 x 4096 x 4096 (4, 5, 7) 94.2 / 94.1 / 94.2; 4104 x 4096 x 1336
+// (4, 6, 8) 50 / 56 / 64. With an MN-major B narrow tiles gain less (half of a 64-column box is not used at 192): 1333 x 4104 x
+// 4096 51.2 / 49.2 / 47.1, 1333 x 4096 x 4104 51.2 / 57.3 / 59.4, 4104 x 4096 x 1336 41.8 / 56.1 / 54.2.
+static int pair_tile_n(int M, int N, int pairs, bool b_mn) {
+  const long long num_m = (M + 255) / 256;
+  auto cost = [&](int bn, double per_col) {
+    const long long tiles = num_m * ((N + bn - 1) / bn);
+    return (double)((tiles + pairs - 1) / pairs) * (bn * per_col);
+  };
+  int best = 256;
+  double c = cost(256, 1.0);
+  if (cost(192, b_mn ? 1.4 : 1.09) < c) { best = 192; c = cost(192, b_mn ? 1.4 : 1.09); }
+  if (cost(128, b_mn ? 1.4 : 1.16) < c) best = 128;
+  return best;
+}
+
+template <int EPI, bool OUT_F32, bool A_MN, bool B_MN, int BN>
+static int launch_pair_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int ctas, cudaStream_t stream) {
+  if constexpr (!OUT_F32) {
+    if (p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
+      GemmOutMaps om;
+      int rc = encode_tmap_2d(&om.m[0], kTmapBf16, p.C, (uint64_t)p.N, (uint64_t)p.M, (uint64_t)p.ldc * 2, 64, 32, kSwizzle128);
+      if (rc) return rc;
+      auto kern = gemm_umma2_tma_kernel<EPI, A_MN, B_MN, BN>;
+      PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemm2SmemTotal));
+      kern<<<ctas, kGemmThreads, kGemm2SmemTotal, stream>>>(ta, tb, om, p);
+      PKB_CHECK_CUDA(cudaGetLastError());
+      return kApiOk;
+    }
+  }
+  auto launch = [&](auto kern) -> int {
+    PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemm2SmemTotal));
+    kern<<<ctas, kGemmThreads, kGemm2SmemTotal, stream>>>(ta, tb, p);
+    PKB_CHECK_CUDA(cudaGetLastError());
+    return kApiOk;
+  };
+  if constexpr (A_MN || B_MN) return launch(gemm_umma2_mn_kernel<EPI, OUT_F32, A_MN, B_MN, BN>);
+  else return launch(gemm_umma2_kernel<EPI, OUT_F32, BN>);
+}
+
+// 256 x BN tiles on clusters of two CTAs (every operand byte crosses L2 -> shared memory once per pair). `a` / `b` are K-major
+// unless A_MN / B_MN; num_ctas 0 = all SMs.
 template <int EPI, bool OUT_F32, bool A_MN, bool B_MN>
-static int launch_pair_mn(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int M, int N, cudaStream_t stream) {
-  auto kern = gemm_umma2_mn_kernel<EPI, OUT_F32, A_MN, B_MN>;
-  PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemm2SmemTotal));
+static int launch_pair(const CUtensorMap& ta, const void* b, long long ldb, GemmParams p, int num_ctas, cudaStream_t stream) {
   p.group_m = 8;
-  const int tiles = ((M + 255) / 256) * ((N + 255) / 256);
-  int ctas = sm_count() & ~1;
+  int ctas = (num_ctas > 0 ? num_ctas : sm_count()) & ~1;
+  const int bn = pair_tile_n(p.M, p.N, ctas / 2, B_MN);
+  const int tiles = ((p.M + 255) / 256) * ((p.N + bn - 1) / bn);
   if (ctas > 2 * tiles) ctas = 2 * tiles;
-  kern<<<ctas, kGemmThreads, kGemm2SmemTotal, stream>>>(ta, tb, p);
-  PKB_CHECK_CUDA(cudaGetLastError());
+  CUtensorMap tb;
+  int rc = B_MN ? encode_tmap_2d(&tb, kTmapBf16, b, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)ldb * 2, 64, kGemmBlockK, kSwizzle128)
+                : encode_tmap_2d(&tb, kTmapBf16, b, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldb * 2, kGemmBlockK, (uint32_t)bn / 2, kSwizzle128);
+  if (rc) return rc;
+  if (bn == 128) return launch_pair_bn<EPI, OUT_F32, A_MN, B_MN, 128>(ta, tb, p, ctas, stream);
+  if (bn == 192) return launch_pair_bn<EPI, OUT_F32, A_MN, B_MN, 192>(ta, tb, p, ctas, stream);
+  return launch_pair_bn<EPI, OUT_F32, A_MN, B_MN, 256>(ta, tb, p, ctas, stream);
+}
+
+template <bool OUT_F32>
+static int dispatch_pair(int epi, const CUtensorMap& ta, const void* b, long long ldb, const GemmParams& p, int num_ctas,
+                         cudaStream_t stream) {
+  switch (epi) {
+    case kEpiNone: return launch_pair<kEpiNone, OUT_F32, false, false>(ta, b, ldb, p, num_ctas, stream);
+    case kEpiSilu: return launch_pair<kEpiSilu, OUT_F32, false, false>(ta, b, ldb, p, num_ctas, stream);
+    case kEpiBias: return launch_pair<kEpiBias, OUT_F32, false, false>(ta, b, ldb, p, num_ctas, stream);
+    case kEpiBiasSilu: return launch_pair<kEpiBiasSilu, OUT_F32, false, false>(ta, b, ldb, p, num_ctas, stream);
+  }
+  set_last_error("unknown epilogue");
+  return kApiBadArgument;
+}
+
+// Up to 64 rows and at most one 128-column tile per SM: the kernel that shares a tile's K range between the CTAs of a cluster
+// (gemm_split.cuh). Measured against one CTA per tile, L2 flushed, us: 33 x 1024 x 8192 15.2 / 33.7, 7 x 264 x 16384 15.5 / 57.3,
+// 17 x 4096 x 14336 33.8 / 60.4, 1 x 14336 x 4096 33.7 / 44.0, 16 x 14336 x 4096 35.7 / 37.8, 64 x 256 x 256 9.2 / 9.2; with more
+// rows the exchange of 128-row partial sums costs what the shorter K range gives: 100 x 2048 x 2048 21.5 / 15.5.
+static bool split_fits(int M, int N) {
+  return M <= 64 && (N + 127) / 128 <= sm_count();
+}
+
+// Cluster size: as many CTAs as leave every tile's cluster resident at once (a GPC holds 16 to 20 SMs: 16 clusters of 8, 32 of 4,
+// 64 of 2), and at least four K blocks each.
+static int split_count(int tiles, int num_k) {
+  int s = tiles <= 16 ? 8 : tiles <= 32 ? 4 : tiles <= 64 ? 2 : 1;
+  while (s > 1 && num_k < 4 * s) s >>= 1;
+  return s;
+}
+
+template <int EPI, bool OUT_F32, bool B_MN>
+static int launch_split(const void* a, long long lda, const void* b, long long ldb, const GemmParams& p, cudaStream_t stream) {
+  const int a_rows = p.M <= 16 ? 16 : p.M <= 32 ? 32 : 64;
+  int stages = kSplitRingBytes / (a_rows * 128 + kSplitBN * 128);
+  if (stages > kSplitMaxStages) stages = kSplitMaxStages;
+  CUtensorMap ta, tb;
+  int rc = encode_tmap_2d(&ta, kTmapBf16, a, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)lda * 2, kGemmBlockK, (uint32_t)a_rows, kSwizzle128);
+  if (rc) return rc;
+  rc = B_MN ? encode_tmap_2d(&tb, kTmapBf16, b, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)ldb * 2, 64, kGemmBlockK, kSwizzle128)
+            : encode_tmap_2d(&tb, kTmapBf16, b, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldb * 2, kGemmBlockK, kSplitBN, kSwizzle128);
+  if (rc) return rc;
+  const int tiles = (p.N + kSplitBN - 1) / kSplitBN;
+  const int splits = split_count(tiles, (p.K + kGemmBlockK - 1) / kGemmBlockK);
+  auto kern = gemm_split_kernel<EPI, OUT_F32, B_MN>;
+  PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemTotal));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * splits));
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.dynamicSmemBytes = kSplitSmemTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  PKB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, p, splits, a_rows, stages));
   return kApiOk;
+}
+
+template <bool OUT_F32>
+static int dispatch_split(int epi, const void* a, long long lda, const void* b, long long ldb, const GemmParams& p, cudaStream_t stream) {
+  switch (epi) {
+    case kEpiNone: return launch_split<kEpiNone, OUT_F32, false>(a, lda, b, ldb, p, stream);
+    case kEpiSilu: return launch_split<kEpiSilu, OUT_F32, false>(a, lda, b, ldb, p, stream);
+    case kEpiBias: return launch_split<kEpiBias, OUT_F32, false>(a, lda, b, ldb, p, stream);
+    case kEpiBiasSilu: return launch_split<kEpiBiasSilu, OUT_F32, false>(a, lda, b, ldb, p, stream);
+  }
+  set_last_error("unknown epilogue");
+  return kApiBadArgument;
 }
 
 }  // namespace pkb
@@ -114,12 +186,8 @@ extern "C" int pkb_gemm_bf16_pair(const void* a, long long lda, const void* b, l
   PKB_CHECK_ARG(M > 0 && N > 0 && K > 0, "empty problem");
   PKB_CHECK_ARG(lda % 8 == 0 && ldb % 8 == 0 && K % 8 == 0, "lda, ldb, K must be multiples of 8");
   PKB_CHECK_ARG((epilogue & 2) == 0 || bias != nullptr, "bias epilogue without bias");
-  CUtensorMap ta, tb;
-  int rc = encode_tmap_2d(&ta, kTmapBf16, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2,
-                          kGemmBlockK, 128, kSwizzle128);
-  if (rc) return rc;
-  rc = encode_tmap_2d(&tb, kTmapBf16, b, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, kGemmBlockK,
-                      128, kSwizzle128);
+  CUtensorMap ta;
+  int rc = encode_tmap_2d(&ta, kTmapBf16, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, kGemmBlockK, 128, kSwizzle128);
   if (rc) return rc;
   GemmParams p = {};
   p.M = M; p.N = N; p.K = K;
@@ -128,23 +196,10 @@ extern "C" int pkb_gemm_bf16_pair(const void* a, long long lda, const void* b, l
   p.alpha = alpha;
   p.status = status_block_device_ptr();
   p.wait_budget_ns = kDefaultWaitBudgetNs;
-  p.group_m = 8;
   p.kernel_id = 101;
   p.world = 1;
-  const int tiles = ((M + 255) / 256) * ((N + 255) / 256);
-  int ctas = num_ctas > 0 ? num_ctas : sm_count();
-  ctas &= ~1;
-  if (ctas > 2 * tiles) ctas = 2 * tiles;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (!out_f32 && ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0) {
-    GemmOutMaps om;
-    rc = encode_tmap_2d(&om.m[0], kTmapBf16, c, (uint64_t)N, (uint64_t)M, (uint64_t)ldc * 2, 64, 32,
-                        kSwizzle128);
-    if (rc) return rc;
-    return dispatch_pair_tma(epilogue, ta, tb, om, p, ctas, s);
-  }
-  return out_f32 ? dispatch_pair<true>(epilogue, ta, tb, p, ctas, s)
-                 : dispatch_pair<false>(epilogue, ta, tb, p, ctas, s);
+  return out_f32 ? dispatch_pair<true>(epilogue, ta, b, ldb, p, num_ctas, s) : dispatch_pair<false>(epilogue, ta, b, ldb, p, num_ctas, s);
 }
 
 extern "C" int pkb_gemm_bf16(const void* a, long long lda, const void* b, long long ldb, void* c,
@@ -186,6 +241,29 @@ extern "C" int pkb_gemm_bf16(const void* a, long long lda, const void* b, long l
                    : dispatch_epi<256, false>(epilogue, ta, tb, p, ctas, s);
   return out_f32 ? dispatch_epi<128, true>(epilogue, ta, tb, p, ctas, s)
                  : dispatch_epi<128, false>(epilogue, ta, tb, p, ctas, s);
+}
+
+// The form chosen by shape: few rows -> gemm_split.cuh (see split_fits); from 512 x 256 on the CTA pairs; else
+// one CTA per tile.
+extern "C" int pkb_gemm_bf16_auto(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N,
+                                  int K, const void* bias, float alpha, int epilogue, int out_f32, void* stream) {
+  PKB_CHECK_ARG(M > 0 && N > 0 && K > 0, "empty problem");
+  if (!split_fits(M, N))
+    return M >= 512 && N >= 256 ? pkb_gemm_bf16_pair(a, lda, b, ldb, c, ldc, M, N, K, bias, alpha, epilogue, out_f32, 0, stream)
+                                : pkb_gemm_bf16(a, lda, b, ldb, c, ldc, M, N, K, bias, alpha, epilogue, out_f32, 0, 0, stream);
+  PKB_CHECK_ARG(lda % 8 == 0 && ldb % 8 == 0 && K % 8 == 0, "lda, ldb, K must be multiples of 8");
+  PKB_CHECK_ARG((epilogue & 2) == 0 || bias != nullptr, "bias epilogue without bias");
+  GemmParams p = {};
+  p.M = M; p.N = N; p.K = K;
+  p.C = c; p.ldc = ldc;
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.alpha = alpha;
+  p.status = status_block_device_ptr();
+  p.wait_budget_ns = kDefaultWaitBudgetNs;
+  p.kernel_id = 108;
+  p.world = 1;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return out_f32 ? dispatch_split<true>(epilogue, a, lda, b, ldb, p, s) : dispatch_split<false>(epilogue, a, lda, b, ldb, p, s);
 }
 
 // Grouped (ragged) GEMM: rows of A are grouped back to back, group e = rows
@@ -338,11 +416,16 @@ extern "C" int pkb_gemm_bf16_bkn(const void* a, long long lda, const void* b, lo
   int ctas = sm_count();
   if (ctas > tiles) ctas = tiles;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (pair_mn_enabled() && M >= 256 && N >= 256) {
-    // large problems: 256 x 256 tiles on CTA pairs (every operand byte crosses L2 -> shared memory once per pair)
+  if (split_fits(M, N)) {
+    p.kernel_id = 109;
     if (epilogue == kEpiSilu)
-      return out_f32 ? launch_pair_mn<kEpiSilu, true, false, true>(ta, tb, p, M, N, s) : launch_pair_mn<kEpiSilu, false, false, true>(ta, tb, p, M, N, s);
-    return out_f32 ? launch_pair_mn<kEpiNone, true, false, true>(ta, tb, p, M, N, s) : launch_pair_mn<kEpiNone, false, false, true>(ta, tb, p, M, N, s);
+      return out_f32 ? launch_split<kEpiSilu, true, true>(a, lda, b, ldb, p, s) : launch_split<kEpiSilu, false, true>(a, lda, b, ldb, p, s);
+    return out_f32 ? launch_split<kEpiNone, true, true>(a, lda, b, ldb, p, s) : launch_split<kEpiNone, false, true>(a, lda, b, ldb, p, s);
+  }
+  if (pair_mn_enabled() && M >= 256 && N >= 256) {
+    if (epilogue == kEpiSilu)
+      return out_f32 ? launch_pair<kEpiSilu, true, false, true>(ta, b, ldb, p, 0, s) : launch_pair<kEpiSilu, false, false, true>(ta, b, ldb, p, 0, s);
+    return out_f32 ? launch_pair<kEpiNone, true, false, true>(ta, b, ldb, p, 0, s) : launch_pair<kEpiNone, false, false, true>(ta, b, ldb, p, 0, s);
   }
   constexpr int smem = GemmSmem<128>::kTotal;
 #define PKB_BKN(EPI, F32)                                                                          \
@@ -379,7 +462,7 @@ extern "C" int pkb_gemm_bf16_tn(const void* a, long long lda, const void* b, lon
   if (ctas > tiles) ctas = tiles;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (pair_mn_enabled() && M >= 256 && N >= 256)
-    return out_f32 ? launch_pair_mn<kEpiNone, true, true, true>(ta, tb, p, M, N, s) : launch_pair_mn<kEpiNone, false, true, true>(ta, tb, p, M, N, s);
+    return out_f32 ? launch_pair<kEpiNone, true, true, true>(ta, b, ldb, p, 0, s) : launch_pair<kEpiNone, false, true, true>(ta, b, ldb, p, 0, s);
   constexpr int smem = GemmSmem<256>::kTotal;
   if (out_f32) {
     auto kern = gemm_umma_tn_kernel<256, true>;

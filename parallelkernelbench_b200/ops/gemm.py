@@ -39,6 +39,12 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, *, out: torch.Tensor | None = No
         if bias.dtype != torch.bfloat16 or bias.numel() != N:
             raise ValueError("bias must be bf16 [N]")
     lib = nv.cuda_lib()
+    if mode == "auto" and block_n == 0 and num_ctas == 0:
+        nv.check(lib.pkb_gemm_bf16_auto(nv.ptr(a), nv.c_ll(a.stride(0)), nv.ptr(w), nv.c_ll(w.stride(0)), nv.ptr(out),
+                                        nv.c_ll(out.stride(0)), M, N, K, nv.ptr(bias), nv.c_float(alpha), EPILOGUES[epilogue],
+                                        1 if out.dtype == torch.float32 else 0, nv.current_stream()), "pkb_gemm_bf16_auto")
+        nv.count_launch()
+        return out
     if mode == "auto":
         mode = "pair" if (block_n == 0 and M >= 512 and N >= 256) else "single"
     if mode == "pair":

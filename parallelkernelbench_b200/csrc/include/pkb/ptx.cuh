@@ -245,10 +245,11 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* desc, uint32_t s
 __device__ __forceinline__ void tma_store_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
-// Adds `bytes` of fp32 from shared memory into global memory (16-byte aligned on both sides, a multiple of 16 bytes): one
-// request to the TMA unit instead of bytes / 16 vector reductions issued by threads. Joins the thread's bulk group.
-__device__ __forceinline__ void bulk_reduce_add_f32(void* gdst, uint32_t smem_src, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(gdst), "r"(smem_src), "r"(bytes)
+// out[box] += box: fp32 additions of a tile in shared memory into global memory (one request for the whole box)
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* desc, uint32_t smem_src, int32_t c0, int32_t c1, int32_t c2) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(desc)),
+               "r"(smem_src), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
 template <int N>

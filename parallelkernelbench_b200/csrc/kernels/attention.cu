@@ -1016,7 +1016,7 @@ static_assert(128 * kFa3RegsIo + 256 * kFa3RegsSoftmax + 128 * kFa3RegsCorr <= 6
 // 1540 cycles the exponential loop took.
 // TRACE: CTA (0,0,0) records clock64 at the hand-over points of every role (see fa_trace) - a separate instantiation, so the
 // production kernel carries none of it.
-template <int D, int OPT, bool TRACE = false>
+template <int D, int OPT, bool TRACE = false, int TILES = 2>
 __device__ __forceinline__ void fa_fwd3_cta(const CUtensorMap& tmap_q, const CUtensorMap& tmap_k,
                                             const CUtensorMap& tmap_v, const FaParams& p, const int q_pair,
                                             const int head, const int batch) {
@@ -1049,8 +1049,8 @@ __device__ __forceinline__ void fa_fwd3_cta(const CUtensorMap& tmap_q, const CUt
   const int lane = threadIdx.x & 31;
   const int kv_head = head / (d.hq / d.hkv);
   const int n_q_tiles = (d.sq + kFaTile - 1) / kFaTile;
-  const int qt0 = q_pair * 2;
-  const bool has1 = qt0 + 1 < n_q_tiles;
+  const int qt0 = q_pair * TILES;
+  const bool has1 = TILES == 2 && qt0 + 1 < n_q_tiles;
   const int q_row0 = qt0 * kFaTile;
   const int q_seg = q_row0 / d.q_seg_rows;
   const int q_pos0 = d.q_seg_pos[q_seg] + (q_row0 - q_seg * d.q_seg_rows);   // both tiles lie in one segment
@@ -1440,11 +1440,17 @@ __device__ __forceinline__ void fa_fwd3_cta(const CUtensorMap& tmap_q, const CUt
   }
 }
 
-template <int D, int OPT, bool TRACE = false>
+// TILES = 1: one Q tile per CTA, for problems whose pairs of tiles would leave SMs without a CTA (a tile alone has the
+// exponential unit to itself: 28.7 instead of 33.8 us at batch 2, S = 1024, 8 / 2 heads, d = 128, causal, 64 or 128 CTAs).
+template <int D, int OPT, bool TRACE = false, int TILES = 2>
 __global__ void __launch_bounds__(kFaThreads, 1)
 fa_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
-  fa_fwd3_cta<D, OPT, TRACE>(tmap_q, tmap_k, tmap_v, p, gridDim.x - 1 - blockIdx.x, blockIdx.y, blockIdx.z);
+  // x runs fastest. Causal: x = head, y = Q tiles, so that the long walks of all heads start before any short one (32 / 8 heads,
+  // d = 128: S = 4096 214 -> 182 us, S = 16384 2018 -> 1905 us). Else every walk is as long and the tiles of a head, which read
+  // the same K and V, stay together (S = 3001, d = 64: 165 us, 171 the other way round).
+  const int tiles = p.d.causal ? gridDim.y : gridDim.x, tile = p.d.causal ? blockIdx.y : blockIdx.x;
+  fa_fwd3_cta<D, OPT, TRACE, TILES>(tmap_q, tmap_k, tmap_v, p, tiles - 1 - tile, p.d.causal ? blockIdx.x : blockIdx.y, blockIdx.z);
 }
 
 // ================================================================================================
@@ -2056,15 +2062,18 @@ static int launch_fa(const pkb_attn_desc* desc, const void* q, const void* k, co
     }
   } else if (fa_use_pairs(d) && p.trace != nullptr && fa_use_v3()) {
     constexpr int smem = Fa3Smem<D>::kTotal;
-    dim3 grid((n_tiles + 1) / 2, d.hq, d.batch);
+    const int tiles = (n_tiles + 1) / 2;
+    dim3 grid(d.causal ? d.hq : tiles, d.causal ? tiles : d.hq, d.batch);
     auto kern = fa_fwd3_kernel<D, kFa3DefaultOpt, true>;
     PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     kern<<<grid, kFaThreads, smem, stream>>>(tq, tk, tv, p);
   } else if (fa_use_pairs(d) && p.trace == nullptr && fa_use_v3()) {
     constexpr int smem = Fa3Smem<D>::kTotal;
-    dim3 grid((n_tiles + 1) / 2, d.hq, d.batch);
     // PKB_FA_OPT=0..3 selects the softmax arithmetic variant (bit 0: packed pairs and three-input maxima, bit 1: polynomial)
     static const int opt = [] { const char* e = getenv("PKB_FA_OPT"); return (e != nullptr && e[0] >= '0' && e[0] <= '9') ? atoi(e) : kFa3DefaultOpt; }();
+    const bool one_tile = opt == kFa3DefaultOpt && (long long)n_tiles * d.hq * d.batch <= sm_count();
+    const int tiles = one_tile ? n_tiles : (n_tiles + 1) / 2;
+    dim3 grid(d.causal ? d.hq : tiles, d.causal ? tiles : d.hq, d.batch);
 #define PKB_FA3(O)                                                                                   \
     {                                                                                                \
       auto kern = fa_fwd3_kernel<D, O>;                                                              \
@@ -2072,7 +2081,13 @@ static int launch_fa(const pkb_attn_desc* desc, const void* q, const void* k, co
       kern<<<grid, kFaThreads, smem, stream>>>(tq, tk, tv, p);                                       \
     }
     switch (opt) {
-      case 1: PKB_FA3(1) break;
+      case 1:
+        if (one_tile) {
+          auto kern = fa_fwd3_kernel<D, 1, false, 1>;
+          PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+          kern<<<grid, kFaThreads, smem, stream>>>(tq, tk, tv, p);
+        } else PKB_FA3(1)
+        break;
       case 2: PKB_FA3(2) break;
       case 3: PKB_FA3(3) break;
       case 5: PKB_FA3(5) break;

@@ -223,7 +223,6 @@ extern "C" int pkb_decoder_layer_bwd(const pkb_layer_desc* L, const void* x, con
   float* dq = static_cast<float*>(b.dqkv32);
   float* dk = dq + b.dq_elems;
   float* dv = dk + b.dk_elems;
-  PKB_CHECK_CUDA(cudaMemsetAsync(dq, 0, (size_t)(b.dq_elems + 2 * b.dk_elems) * 4, static_cast<cudaStream_t>(st)));
   PKB_TRY(pkb_flash_attn_bwd(&ad, s.q, s.k, s.v, s.att, b.datt, s.lse, b.delta, b.lse2, dq, dk, dv, st));
   PKB_TRY(pkb_qkv_rope_merge(dq, dk, dv, cos_t, sin_t, b.dqkv, S, L->hq, L->hkv, d, st));
   PKB_TRY(linear_dx(b.dqkv, at(params, p.wqkv), b.dh, S, QKV, H, st));

@@ -215,9 +215,9 @@ def case_fa_trace(t: _Timer) -> dict:
 def case_fa_bwd_trace(t: _Timer) -> dict:
     """Device-side timeline of the attention backward's heaviest CTA (the first KV tile, which every query tile sees): medians
     of the intervals between consecutive stamps of each role over the steady steps, in SM cycles. Roles: 0 issuing warp
-    (0 step start, 1 Q/dO landed, 2 dQ drained, 3 S and dP issued, 4 P and dS in shared memory, 5 dV and dK issued, 6 dQ issued),
-    1 P / dS warps (0 start, 1 S and dP complete, 2 previous P/dS consumed, 3 computed, 4 published), 2 dQ drain warps
-    (0 start, 1 dQ complete, 2 drained)."""
+    (0 step start, 1 dO landed, 2 dQ of the step before drained, 3 dP issued, 4 P in shared memory, 5 dV and the next S issued and
+    dS in shared memory, 6 dQ and dK issued), 1 P / dS warps (0 start, 1 S complete, 2 P published, 3 dP complete, 4 dS published),
+    2 dQ drain warps (0 start, 1 dQ complete, 2 drained)."""
     from .. import _native as nv
     from ..ops.attention import flash_attn_bwd, flash_attn_fwd
 

@@ -230,7 +230,7 @@ class RingAttention:
         qc, oc, doc = (t.contiguous() for t in (q, out, dout))
         lsec = lse.reshape(1, self.hq, self.rows).float().contiguous()
         delta, lse2 = torch.empty_like(lsec), torch.empty_like(lsec)
-        dq = torch.zeros((self.rows, self.hq, self.D), dtype=torch.float32, device=q.device)
+        dq = torch.empty((self.rows, self.hq, self.D), dtype=torch.float32, device=q.device)
         nv.check(nv.cuda_lib().pkb_flash_attn_bwd_scatter(ctypes.byref(d), nv.ptr(qc), nv.ptr(kg), nv.ptr(vg), nv.ptr(oc), nv.ptr(doc),
                                                           nv.ptr(lsec), nv.ptr(delta), nv.ptr(lse2), nv.ptr(dq), dk_ptrs, dv_ptrs,
                                                           nv.current_stream()), "pkb_flash_attn_bwd_scatter")
@@ -246,7 +246,7 @@ def flash_attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch
     """Attention backward from a saved forward. ``q, out, dout`` [Sq, Hq, D] (or [B, Sq, Hq, D]); ``k, v`` [Skv, Hkv, D]
     (or with the batch dimension); ``lse`` [Hq, Sq] (or [B, Hq, Sq]), natural log. Positions are described as in
     :func:`flash_attn_fwd`; without segment lists query row i sits at ``q_pos0 + i`` and key row j at j.
-    ``dk_out`` / ``dv_out``: optional fp32 tensors shaped like k / v that receive the result (they are zero-filled here);
+    ``dk_out`` / ``dv_out``: optional fp32 tensors shaped like k / v that receive the result;
     a caller that reduces them over ranks passes symmetric-heap tensors so that the collective needs no staging copy.
     Returns fp32 ``(dq, dk, dv)`` shaped like q, k, v. bf16 inputs with head dimension 64 or 128 run on the tcgen05
     kernel (dK/dV accumulate in TMEM, dQ by fp32 vector reductions); anything else takes the PyTorch restatement."""
@@ -295,9 +295,9 @@ def flash_attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch
         lsec = lse.float().contiguous()
         delta = torch.empty_like(lsec)
         lse2 = torch.empty_like(lsec)
-        dq = torch.zeros(q.shape, dtype=torch.float32, device=q.device)
-        dk = dk_out.view(k.shape).zero_() if dk_out is not None else torch.zeros(k.shape, dtype=torch.float32, device=q.device)
-        dv = dv_out.view(v.shape).zero_() if dv_out is not None else torch.zeros(v.shape, dtype=torch.float32, device=q.device)
+        dq = torch.empty(q.shape, dtype=torch.float32, device=q.device)
+        dk = dk_out.view(k.shape) if dk_out is not None else torch.empty(k.shape, dtype=torch.float32, device=q.device)
+        dv = dv_out.view(v.shape) if dv_out is not None else torch.empty(v.shape, dtype=torch.float32, device=q.device)
         nv.check(nv.cuda_lib().pkb_flash_attn_bwd(ctypes.byref(d), nv.ptr(qc), nv.ptr(kc), nv.ptr(vc), nv.ptr(oc), nv.ptr(doc), nv.ptr(lsec),
                                                   nv.ptr(delta), nv.ptr(lse2), nv.ptr(dq), nv.ptr(dk), nv.ptr(dv), nv.current_stream()),
                  "pkb_flash_attn_bwd")

@@ -1,0 +1,42 @@
+"""Attention backward whose KV tiles are shared by several CTAs, and what it writes where no query looks."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,sq,skv,hq,hkv,D,causal", [(1, 130, 130, 8, 1, 64, True), (2, 1000, 1000, 4, 1, 128, True), (1, 64, 700, 2, 2, 128, False),
+                                                      (1, 2000, 129, 6, 3, 64, False), (1, 100, 900, 1, 1, 64, True), (1, 300, 2000, 16, 16, 128, True),
+                                                      (4, 257, 257, 16, 8, 128, True)])
+def test_attention_backward_shared_between_ctas(B, sq, skv, hq, hkv, D, causal):
+    """dK / dV are then added up in global memory, so stale values in the buffers would show: they are filled with NaN first."""
+    from parallelkernelbench_b200.ops.attention import flash_attn_bwd, flash_attn_fwd
+    from parallelkernelbench_b200.refs.attention import attention_bwd_positions_ref
+
+    torch.manual_seed(5)
+    q, dout = (torch.randn(B, sq, hq, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(B, skv, hkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    out, lse = flash_attn_fwd(q, k, v, causal=causal)
+    dk_buf, dv_buf = (torch.full(k.shape, float("nan"), device="cuda") for _ in range(2))
+    dq, dk, dv = flash_attn_bwd(q, k, v, out, lse, dout, causal=causal, dk_out=dk_buf, dv_out=dv_buf)
+    q_pos, kv_pos = torch.arange(sq, device="cuda"), torch.arange(skv, device="cuda")
+    for b in range(B):
+        ref = attention_bwd_positions_ref(q[b], k[b], v[b], out[b], lse[b], dout[b], q_pos, kv_pos, causal, D ** -0.5)
+        for name, got, r in zip(("dq", "dk", "dv"), (dq[b], dk[b], dv[b]), ref):
+            err = (got - r).abs().max().item()
+            assert err <= 2e-2 * max(r.abs().max().item(), 1.0), f"{name}: {err}"      # bf16 P and dS, as in test_gpu_attention
+
+
+@pytest.mark.parametrize("splits", [False, True])
+def test_attention_backward_zeroes_rows_outside_all_segments(splits):
+    from parallelkernelbench_b200.ops.attention import flash_attn_bwd, flash_attn_fwd
+
+    hq, hkv, D, C = (8, 1, 64, 128) if splits else (8, 8, 64, 2560)
+    q = torch.randn(1, C, hq, D, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(1, 3 * C, hkv, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    seg = [(C, 0, C)]                                                     # the middle third of the buffer
+    out, lse = flash_attn_fwd(q, k, v, causal=True, kv_segments=seg)
+    bufs = [torch.full(k.shape, float("nan"), device="cuda") for _ in range(2)]
+    _, dk, dv = flash_attn_bwd(q, k, v, out, lse, torch.randn_like(q), causal=True, kv_segments=seg, dk_out=bufs[0], dv_out=bufs[1])
+    for g in (dk, dv):
+        assert (g[:, :C] == 0).all() and (g[:, 2 * C:] == 0).all() and torch.isfinite(g).all() and (g[:, C:2 * C] != 0).any()

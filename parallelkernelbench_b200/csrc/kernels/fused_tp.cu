@@ -130,7 +130,7 @@ __device__ __forceinline__ void ag_push_role(const TpAgArgs& a) {
   }
 }
 
-template <int EPI>
+template <int EPI, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 tp_ag_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                   const __grid_constant__ CUtensorMap tmap_b,
@@ -141,9 +141,8 @@ tp_ag_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     ag_push_role(a);
     return;
   }
-  gemm_umma2_cta<EPI, false, true, false, true>(tmap_a, tmap_b, p, (blockIdx.x - a.comm_ctas) >> 1,
-                                                (gridDim.x - a.comm_ctas) >> 1, &out_maps,
-                                                &tmap_a_local);
+  gemm_umma2_cta<EPI, false, true, false, true, false, false, false, false, BN>(
+      tmap_a, tmap_b, p, (blockIdx.x - a.comm_ctas) >> 1, (gridDim.x - a.comm_ctas) >> 1, &out_maps, &tmap_a_local);
 }
 
 // Sum of the partial slots of one output row, kept in registers. Thread t owns the 16-byte chunks t, t + T, t + 2T, ... of
@@ -185,16 +184,18 @@ struct TpRsArgs {
   int rows_per_rank;
 };
 
+template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 tp_gemm_rs_rmsnorm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                           const __grid_constant__ CUtensorMap tmap_b,
                           const __grid_constant__ GemmOutMaps out_maps, const GemmParams p,
                           const TpRsArgs a) {
   const SymmCtx& c = a.ctx;
-  // all ranks have entered this call => all ranks have consumed the previous call's receive slots
-  if (!cluster_pair_all(symm_block_barrier(c, 301, 1))) return;
-  gemm_umma2_cta<kEpiNone, false, false, true, true>(tmap_a, tmap_b, p, blockIdx.x >> 1,
-                                                     gridDim.x >> 1, &out_maps);
+  // all ranks have entered this call => all ranks have consumed the previous call's receive slots (a rank by itself: its
+  // previous kernel has)
+  if (c.gsize > 1 && !cluster_pair_all(symm_block_barrier(c, 301, 1))) return;
+  gemm_umma2_cta<kEpiNone, false, false, true, true, false, false, false, false, BN>(tmap_a, tmap_b, p, blockIdx.x >> 1,
+                                                                                     gridDim.x >> 1, &out_maps);
   __syncthreads();
 
   // ---- consumer phase: reduce the W partial slots of my rows and normalise --------------------
@@ -465,6 +466,13 @@ int pkb_tp_ag_gemm_set_wait_stats(void* dev_words) {
 
 // Default number of communication CTAs of the all-gather -> GEMM kernel for a group of `world` ranks (bulk_push: the TMA bulk
 // ring; otherwise the thread-copy push). Exposed so that the rule can be checked without a GPU.
+// Width of the CTA pairs' tiles: 128 columns where tiles of 256 would leave half of the pairs without one (the same on every
+// rank: it follows from the shapes alone).
+static int tp_tile_n(int M, int N) {
+  const long long tiles = (long long)((M + kGemm2TileM - 1) / kGemm2TileM) * ((N + 255) / 256);
+  return 4 * tiles <= sm_count() ? 128 : 256;
+}
+
 extern "C" int pkb_tp_default_comm_ctas(int world, int bulk_push) {
   if (world <= 1) return 2;
   if (bulk_push) return world >= 8 ? 16 : (world > 4 ? 12 : 8);
@@ -496,7 +504,8 @@ int pkb_tp_ag_gemm(const pkb_symm_ctx* h, const void* x_local, int rows, int K,
   int rc = encode_tmap_2d(&ta, kTmapBf16, g_local, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2,
                           kGemmBlockK, kGemmBlockM, kSwizzle128);
   if (rc) return rc;
-  rc = encode_tmap_2d(&tb, kTmapBf16, w, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, kGemmBlockK, 128,
+  const int bn = tp_tile_n(M, N);
+  rc = encode_tmap_2d(&tb, kTmapBf16, w, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, kGemmBlockK, (uint32_t)bn / 2,
                       kSwizzle128);
   if (rc) return rc;
   PKB_CHECK_ARG((reinterpret_cast<uintptr_t>(x_local) & 15) == 0, "x_local must be 16-byte aligned");
@@ -548,7 +557,8 @@ int pkb_tp_ag_gemm(const pkb_symm_ctx* h, const void* x_local, int rows, int K,
   // producers wait 169 us per call for 96 MiB of remote rows, 8 CTAs 2 us), and the GEMM consumes one remote shard per
   // 1/W of its run time, so the rate the push needs grows with W while the shard size stays: 8 CTAs cover a 32 MiB shard in
   // 115 us, which is enough up to 4 ranks (175 us per shard of GEMM time) and not at 8 ranks (87 us), where 16 are used.
-  if (comm_ctas <= 0) comm_ctas = pkb_tp_default_comm_ctas(W, a.bulk_push);
+  // A rank by itself has nobody to push to: no communication CTAs, no barrier.
+  if (comm_ctas <= 0) comm_ctas = W == 1 ? 0 : pkb_tp_default_comm_ctas(W, a.bulk_push);
   comm_ctas = (comm_ctas + 1) & ~1;  // whole clusters
   const int sms = sm_count() & ~1;
   PKB_CHECK_ARG(comm_ctas < sms && comm_ctas <= kSymmMaxBlocks, "too many communication CTAs");
@@ -556,17 +566,14 @@ int pkb_tp_ag_gemm(const pkb_symm_ctx* h, const void* x_local, int rows, int K,
 
   constexpr int smem = kGemm2SmemTotal;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (epilogue == kEpiSilu) {
-    auto k = tp_ag_gemm_kernel<kEpiSilu>;
+  auto launch = [&](auto k) -> int {
     PKB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     k<<<sms, kGemmThreads, smem, s>>>(ta, tb, tal, om, p, a);
-  } else {
-    auto k = tp_ag_gemm_kernel<kEpiNone>;
-    PKB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    k<<<sms, kGemmThreads, smem, s>>>(ta, tb, tal, om, p, a);
-  }
-  PKB_CHECK_CUDA(cudaGetLastError());
-  return kApiOk;
+    PKB_CHECK_CUDA(cudaGetLastError());
+    return kApiOk;
+  };
+  if (epilogue == kEpiSilu) return bn == 128 ? launch(tp_ag_gemm_kernel<kEpiSilu, 128>) : launch(tp_ag_gemm_kernel<kEpiSilu, 256>);
+  return bn == 128 ? launch(tp_ag_gemm_kernel<kEpiNone, 128>) : launch(tp_ag_gemm_kernel<kEpiNone, 256>);
 }
 
 // out[rows_per_rank, N] = RMSNorm( reduce_scatter( a[gsize*rows_per_rank, K] @ w[N, K]^T ) * scale )
@@ -587,11 +594,12 @@ int pkb_tp_gemm_rs_rmsnorm(const pkb_symm_ctx* h, const void* a_mat, long long l
   const int M = W * rows_per_rank;
   SymmCtx ctx = symm_ctx_from_api(h);
 
+  const int bn = tp_tile_n(h->gsize * rows_per_rank, N);
   CUtensorMap ta, tb;
   int rc = encode_tmap_2d(&ta, kTmapBf16, a_mat, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2,
                           kGemmBlockK, kGemmBlockM, kSwizzle128);
   if (rc) return rc;
-  rc = encode_tmap_2d(&tb, kTmapBf16, w, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, kGemmBlockK, 128,
+  rc = encode_tmap_2d(&tb, kTmapBf16, w, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, kGemmBlockK, (uint32_t)bn / 2,
                       kSwizzle128);
   if (rc) return rc;
 
@@ -616,7 +624,7 @@ int pkb_tp_gemm_rs_rmsnorm(const pkb_symm_ctx* h, const void* a_mat, long long l
   while (blocks_per_rank % p.group_m != 0) --p.group_m;
   p.m_block_rotation = ((h->grank + 1) % W) * blocks_per_rank;  // rank+1's rows first, own rows last
 
-  const int num_n = (N + 255) / 256;
+  const int num_n = (N + bn - 1) / bn;
   TpRsArgs a;
   a.ctx = ctx;
   a.recv_off = recv_off; a.done_off = done_off;
@@ -626,7 +634,7 @@ int pkb_tp_gemm_rs_rmsnorm(const pkb_symm_ctx* h, const void* a_mat, long long l
   a.eps = eps; a.scale = scale; a.N = N; a.rows_per_rank = rows_per_rank;
 
   constexpr int smem = kGemm2SmemTotal;
-  auto k = tp_gemm_rs_rmsnorm_kernel;
+  auto k = bn == 128 ? tp_gemm_rs_rmsnorm_kernel<128> : tp_gemm_rs_rmsnorm_kernel<256>;
   PKB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int grid = sm_count() & ~1;
   if (grid > kSymmMaxBlocks) grid = kSymmMaxBlocks;

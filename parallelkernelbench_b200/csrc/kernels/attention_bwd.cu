@@ -664,13 +664,32 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   }
 }
 
-// CTAs per KV tile and head. One, unless the tiles leave half of the SMs without a CTA: then the walk over query heads and Q
-// tiles is shared, at least two steps each, and dK / dV are added up with fp32 reductions (in no fixed order, as dQ always is).
-// Batch 2, S = 1024, 8 / 2 heads, d = 128, causal, 32 tiles on 128 CTAs: 128 -> 39 us.
-static int fa_bwd_splits(long long ctas, int max_steps) {
-  if (ctas <= 0) return 1;
-  long long s = sm_count() / ctas;
-  if (s > max_steps / 2) s = max_steps / 2;
+// CTAs per KV tile and head: as many as bring the longest walk (the first KV tile under a causal mask) down to an SM's share of all
+// steps; at least two steps each, eight where that makes more CTAs than SMs (a CTA's K and V loads and its dK / dV cost about one
+// and a half steps). With more than one, dK / dV are added up with fp32 reductions (in no fixed order, as dQ always is).
+// d = 128, causal: batch 2, S = 1024, 8 / 2 heads (32 tiles) 128 us on one CTA each, 39 us on four, 43 on eight; S = 4096, 16 / 4
+// heads (128 tiles) 334 us on one, 191 on two.
+static int fa_bwd_splits(const pkb_attn_desc& d, int kv_tiles) {
+  const long long rep = d.hq / d.hkv;
+  const long long rows_per_seg = d.num_q_segs == 1 ? d.sq : d.q_seg_rows;
+  const long long q_tiles = (rows_per_seg + kFbTile - 1) / kFbTile;
+  long long total = 0, longest = 0;          // Q tiles that see a KV tile: all KV tiles of a head, and the most of any one
+  for (int s = 0; s < d.num_kv_segs; ++s)
+    for (int t = 0; t * kFbTile < d.kv_seg_len[s]; ++t) {
+      long long seen = 0;
+      for (int q = 0; q < d.num_q_segs; ++q) {
+        const long long hidden = d.causal ? ((long long)d.kv_seg_pos0[s] + t * kFbTile - d.q_seg_pos[q]) / kFbTile : 0;
+        seen += q_tiles - (hidden < 0 ? 0 : hidden > q_tiles ? q_tiles : hidden);
+      }
+      total += seen;
+      if (seen > longest) longest = seen;
+    }
+  const long long heads = (long long)d.hkv * d.batch, sms = sm_count();
+  if (total == 0) return 1;
+  long long s = longest * sms / (total * heads);
+  const long long most = longest * rep;
+  if (s * kv_tiles * heads > sms && s > most / 8) s = most / 8 > sms / (kv_tiles * heads) ? most / 8 : sms / (kv_tiles * heads);
+  if (s > most / 2) s = most / 2;
   return s < 1 ? 1 : (int)s;
 }
 
@@ -701,7 +720,7 @@ static int launch_fa_bwd(const pkb_attn_desc& d, const void* q, const void* k, c
     kv_rows += d.kv_seg_len[s];
   }
   const bool scatter = dk_seg != nullptr && dv_seg != nullptr;
-  const int splits = scatter ? 1 : fa_bwd_splits(kv_tiles * d.hkv * d.batch, (d.sq + kFbTile - 1) / kFbTile * (d.hq / d.hkv));
+  const int splits = scatter ? 1 : fa_bwd_splits(d, kv_tiles);
   // every row of dK / dV is written by the main kernel unless rows lie outside all segments or CTAs add to them
   const long long kv_elems = !scatter && (splits > 1 || kv_rows < d.skv) ? (long long)d.batch * d.skv * d.hkv * D : 0;
   CUtensorMap tdq;

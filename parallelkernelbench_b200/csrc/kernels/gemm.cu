@@ -85,7 +85,7 @@ static int launch_pair_bn(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
 }
 
 // 256 x BN tiles on clusters of two CTAs (every operand byte crosses L2 -> shared memory once per pair). `a` / `b` are K-major
-// unless A_MN / B_MN; num_ctas 0 = all SMs.
+// unless A_MN / B_MN; num_ctas 0 = all SMs, else at least 2 (rounded down to whole pairs).
 template <int EPI, bool OUT_F32, bool A_MN, bool B_MN>
 static int launch_pair(const CUtensorMap& ta, const void* b, long long ldb, GemmParams p, int num_ctas, cudaStream_t stream) {
   p.group_m = 8;
@@ -186,6 +186,7 @@ extern "C" int pkb_gemm_bf16_pair(const void* a, long long lda, const void* b, l
   PKB_CHECK_ARG(M > 0 && N > 0 && K > 0, "empty problem");
   PKB_CHECK_ARG(lda % 8 == 0 && ldb % 8 == 0 && K % 8 == 0, "lda, ldb, K must be multiples of 8");
   PKB_CHECK_ARG((epilogue & 2) == 0 || bias != nullptr, "bias epilogue without bias");
+  PKB_CHECK_ARG(num_ctas != 1, "num_ctas = 1: the tiles of this form belong to pairs of CTAs");
   CUtensorMap ta;
   int rc = encode_tmap_2d(&ta, kTmapBf16, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, kGemmBlockK, 128, kSwizzle128);
   if (rc) return rc;

@@ -142,3 +142,15 @@ def test_default_number_of_push_ctas_follows_the_rank_count():
     assert [f(w, 1) for w in (1, 2, 4, 6, 8)] == [2, 8, 8, 12, 16]
     assert [f(w, 0) for w in (1, 2, 4, 8)] == [2, 8, 8, 16]
     assert all(f(w, b) % 2 == 0 for w in range(1, 9) for b in (0, 1))          # whole CTA pairs
+
+
+def test_pair_gemm_refuses_a_single_cta():
+    """One CTA is no pair: the call is refused before anything is divided by the number of pairs."""
+    import ctypes
+
+    from parallelkernelbench_b200 import _native as nv
+
+    lib = nv.cuda_lib()
+    buf, ll = ctypes.c_void_p(4096), ctypes.c_longlong
+    rc = lib.pkb_gemm_bf16_pair(buf, ll(64), buf, ll(64), buf, ll(256), 512, 256, 64, None, ctypes.c_float(1), 0, 0, 1, None)
+    assert rc != 0 and b"num_ctas" in lib.pkb_last_error()

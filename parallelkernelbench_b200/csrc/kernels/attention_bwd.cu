@@ -779,6 +779,8 @@ extern "C" int pkb_flash_attn_bwd(const pkb_attn_desc* desc, const void* q, cons
   for (int s = 0; s < d.num_kv_segs; ++s)
     PKB_CHECK_ARG(d.kv_seg_row0[s] >= 0 && d.kv_seg_len[s] >= 0 && d.kv_seg_row0[s] + d.kv_seg_len[s] <= d.skv,
                   "kv segment outside the buffer");
+  // the other tensors are held to this by their tensor maps
+  PKB_CHECK_ARG((((uintptr_t)o | (uintptr_t)dk | (uintptr_t)dv) & 15) == 0, "o, dk and dv must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (d.head_dim == 128) return launch_fa_bwd<128>(d, q, k, v, o, dout, lse, delta_scratch, lse2_scratch, dq, dk, dv, s);
   return launch_fa_bwd<64>(d, q, k, v, o, dout, lse, delta_scratch, lse2_scratch, dq, dk, dv, s);
@@ -803,6 +805,7 @@ extern "C" int pkb_flash_attn_bwd_scatter(const pkb_attn_desc* desc, const void*
                   "kv segment outside the buffer");
     PKB_CHECK_ARG(dk_seg[s] != 0 && dv_seg[s] != 0 && ((dk_seg[s] | dv_seg[s]) & 15) == 0, "segment destinations must be 16-byte aligned");
   }
+  PKB_CHECK_ARG(((uintptr_t)o & 15) == 0, "o must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (d.head_dim == 128)
     return launch_fa_bwd<128>(d, q, k, v, o, dout, lse, delta_scratch, lse2_scratch, dq, nullptr, nullptr, s, dk_seg, dv_seg);

@@ -64,6 +64,12 @@ def flash_attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal:
     return out, lse
 
 
+def _aligned16(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and on a 16-byte boundary: a contiguous view may start anywhere, and the kernels read 16 bytes at a time."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def zigzag_positions(world: int, rank: int, chunk: int) -> list[int]:
     """Global start positions of the two chunks a rank owns in the load-balanced causal layout:
     the sequence is cut into ``2 * world`` chunks and rank r holds chunks r and 2*world-1-r."""
@@ -227,7 +233,7 @@ class RingAttention:
             owner = self.group.members[src]
             dk_ptrs[i] = (heap.base + owner * heap.stride + dk_acc.offset) + sgi * seg_bytes
             dv_ptrs[i] = (heap.base + owner * heap.stride + dv_acc.offset) + sgi * seg_bytes
-        qc, oc, doc = (t.contiguous() for t in (q, out, dout))
+        qc, oc, doc = q.contiguous(), _aligned16(out), dout.contiguous()
         lsec = lse.reshape(1, self.hq, self.rows).float().contiguous()
         delta, lse2 = torch.empty_like(lsec), torch.empty_like(lsec)
         dq = torch.empty((self.rows, self.hq, self.D), dtype=torch.float32, device=q.device)
@@ -291,7 +297,7 @@ def flash_attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch
         d.num_kv_segs = len(kv_segments)
         for i, (row0, pos0, ln) in enumerate(kv_segments):
             d.kv_seg_row0[i], d.kv_seg_pos0[i], d.kv_seg_len[i] = row0, pos0, ln
-        qc, kc, vc, oc, doc = (t.contiguous() for t in (q, k, v, out, dout))
+        qc, kc, vc, oc, doc = q.contiguous(), k.contiguous(), v.contiguous(), _aligned16(out), dout.contiguous()
         lsec = lse.float().contiguous()
         delta = torch.empty_like(lsec)
         lse2 = torch.empty_like(lsec)

@@ -154,3 +154,23 @@ def test_pair_gemm_refuses_a_single_cta():
     buf, ll = ctypes.c_void_p(4096), ctypes.c_longlong
     rc = lib.pkb_gemm_bf16_pair(buf, ll(64), buf, ll(64), buf, ll(256), 512, 256, 64, None, ctypes.c_float(1), 0, 0, 1, None)
     assert rc != 0 and b"num_ctas" in lib.pkb_last_error()
+
+
+@pytest.mark.parametrize("moved", ["o", "dk", "dv"])
+def test_attention_backward_refuses_tensors_off_the_16_byte_boundary(moved):
+    """The kernel reads o and writes dk / dv 16 bytes at a time and no tensor map checks them. Refused before any launch."""
+    import ctypes
+
+    from parallelkernelbench_b200 import _native as nv
+    from parallelkernelbench_b200.ops.attention import AttnDesc
+
+    d = AttnDesc()
+    d.batch, d.sq, d.skv, d.hq, d.hkv, d.head_dim, d.causal, d.scale = 1, 128, 128, 1, 1, 64, 1, 0.125
+    d.q_seg_rows, d.num_q_segs, d.num_kv_segs, d.kv_seg_len[0] = 128, 1, 1, 128
+    at = {n: ctypes.c_void_p(4096 + (2 if n == moved else 0)) for n in ("q", "k", "v", "o", "dout", "lse", "delta", "lse2", "dq", "dk", "dv")}
+    lib = nv.cuda_lib()
+    assert lib.pkb_flash_attn_bwd(ctypes.byref(d), *at.values(), None) != 0 and b"aligned" in lib.pkb_last_error()
+    if moved == "o":
+        seg = (ctypes.c_ulonglong * 16)(*[4096] * 16)
+        args = [at[n] for n in ("q", "k", "v", "o", "dout", "lse", "delta", "lse2", "dq")]
+        assert lib.pkb_flash_attn_bwd_scatter(ctypes.byref(d), *args, seg, seg, None) != 0 and b"aligned" in lib.pkb_last_error()

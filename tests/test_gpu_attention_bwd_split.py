@@ -40,3 +40,14 @@ def test_attention_backward_zeroes_rows_outside_all_segments(splits):
     _, dk, dv = flash_attn_bwd(q, k, v, out, lse, torch.randn_like(q), causal=True, kv_segments=seg, dk_out=bufs[0], dv_out=bufs[1])
     for g in (dk, dv):
         assert (g[:, :C] == 0).all() and (g[:, 2 * C:] == 0).all() and torch.isfinite(g).all() and (g[:, C:2 * C] != 0).any()
+
+
+def test_attention_backward_takes_an_output_off_the_16_byte_boundary():
+    from parallelkernelbench_b200.ops.attention import flash_attn_bwd, flash_attn_fwd
+
+    q, k, v, dout = (torch.randn(1, 200, 2, 64, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    out, lse = flash_attn_fwd(q, k, v, causal=True)
+    moved = torch.empty(out.numel() + 1, device="cuda", dtype=torch.bfloat16)[1:].view(out.shape).copy_(out)
+    assert moved.is_contiguous() and moved.data_ptr() % 16 == 2
+    for a, b in zip(flash_attn_bwd(q, k, v, out, lse, dout, causal=True), flash_attn_bwd(q, k, v, moved, lse, dout, causal=True)):
+        assert torch.equal(a, b)

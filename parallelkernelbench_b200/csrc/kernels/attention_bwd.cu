@@ -693,6 +693,21 @@ static int fa_bwd_splits(const pkb_attn_desc& d, int kv_tiles) {
   return s < 1 ? 1 : (int)s;
 }
 
+// KV rows of the buffer that lie in a segment (segments may overlap, so their lengths do not add up to it).
+static int fa_bwd_covered(const pkb_attn_desc& d) {
+  int covered = 0;
+  for (int end = 0;;) {                    // `end`: everything below is counted or outside; the next segment piece starts at `from`
+    int from = d.skv, to = d.skv;
+    for (int s = 0; s < d.num_kv_segs; ++s) {
+      const int a = d.kv_seg_row0[s], b = a + d.kv_seg_len[s];
+      if (b > end && (a > end ? a : end) < from) { from = a > end ? a : end; to = b; }
+    }
+    if (from == d.skv) return covered;
+    covered += to - from;
+    end = to;
+  }
+}
+
 // Trace buffer of the next backward launches (device memory, 3 * kFbTraceSteps * 8 int64, zeroed by the caller); null = off.
 static long long* g_fb_trace = nullptr;
 
@@ -714,15 +729,11 @@ static int launch_fa_bwd(const pkb_attn_desc& d, const void* q, const void* k, c
                       kFbTile, kSwizzle128);
   if (rc) return rc;
   int kv_tiles = 0;
-  long long kv_rows = 0;
-  for (int s = 0; s < d.num_kv_segs; ++s) {
-    kv_tiles += (d.kv_seg_len[s] + kFbTile - 1) / kFbTile;
-    kv_rows += d.kv_seg_len[s];
-  }
+  for (int s = 0; s < d.num_kv_segs; ++s) kv_tiles += (d.kv_seg_len[s] + kFbTile - 1) / kFbTile;
   const bool scatter = dk_seg != nullptr && dv_seg != nullptr;
   const int splits = scatter ? 1 : fa_bwd_splits(d, kv_tiles);
   // every row of dK / dV is written by the main kernel unless rows lie outside all segments or CTAs add to them
-  const long long kv_elems = !scatter && (splits > 1 || kv_rows < d.skv) ? (long long)d.batch * d.skv * d.hkv * D : 0;
+  const long long kv_elems = !scatter && (splits > 1 || fa_bwd_covered(d) < d.skv) ? (long long)d.batch * d.skv * d.hkv * D : 0;
   CUtensorMap tdq;
   rc = encode_tmap_3d(&tdq, kTmapFp32, dq, D, d.hq, (uint64_t)d.batch * d.sq, (uint64_t)D * 4, (uint64_t)d.hq * D * 4, 32, 1, 32,
                       kSwizzle128);

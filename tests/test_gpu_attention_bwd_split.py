@@ -51,3 +51,17 @@ def test_attention_backward_takes_an_output_off_the_16_byte_boundary():
     assert moved.is_contiguous() and moved.data_ptr() % 16 == 2
     for a, b in zip(flash_attn_bwd(q, k, v, out, lse, dout, causal=True), flash_attn_bwd(q, k, v, moved, lse, dout, causal=True)):
         assert torch.equal(a, b)
+
+
+def test_attention_backward_zeroes_uncovered_rows_beside_overlapping_segments():
+    """Two segments over the same rows: their lengths add up to more than the buffer, and a third of it lies outside."""
+    from parallelkernelbench_b200.ops.attention import flash_attn_bwd
+
+    H, D, C = 8, 64, 1280                                                 # 320 tiles: one CTA each
+    q, out, dout = (torch.randn(1, 2 * C, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    k, v = (torch.randn(1, 3 * C, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    lse = torch.full((1, H, 2 * C), 8.0, device="cuda")
+    bufs = [torch.full(k.shape, float("nan"), device="cuda") for _ in range(2)]
+    _, dk, dv = flash_attn_bwd(q, k, v, out, lse, dout, causal=False, kv_segments=[(C, 0, 2 * C), (C, 0, 2 * C)], dk_out=bufs[0], dv_out=bufs[1])
+    for g in (dk, dv):
+        assert (g[:, :C] == 0).all() and torch.isfinite(g).all() and (g[:, C:] != 0).any()

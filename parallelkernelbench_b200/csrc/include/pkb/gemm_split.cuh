@@ -21,12 +21,6 @@ constexpr int kSplitSmemTotal = kSplitRingBytes + 256 + 1024;
 
 constexpr int kSplitPitch = kSplitBN * 4 + 16;    // bytes between rows of partial sums: 16-byte accesses of 8 rows hit all banks
 
-__device__ __forceinline__ float4 ld_shared_cluster_v4(uint32_t cluster_addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
-  return v;
-}
-
 // Epilogue and store of NV (a multiple of 4) neighbouring outputs of one row, the first at column `col` (a multiple of 4) of C.
 template <int EPI, bool OUT_F32, int NV>
 __device__ __forceinline__ void split_store(const GemmParams& p, int row, int col, float (&v)[NV]) {

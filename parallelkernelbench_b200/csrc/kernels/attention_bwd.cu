@@ -1,11 +1,11 @@
 // Flash-attention backward on tcgen05 / TMEM.
 //
-// One CTA owns one 128-row KV tile of one KV head and walks every (query head of the group, 128-row Q tile) pair
-// that can see it. Per pair, from the saved forward (O, log-sum-exp):
+// One CTA, or several that share the walk (see fa_bwd_splits), owns one 128-row KV tile of one KV head and walks every (query head
+// of the group, 128-row Q tile) pair that can see it. Per pair, from the saved forward (O, log-sum-exp):
 //     S  = Q K^T                         (tensor core, TMEM)
 //     dP = dO V^T                        (tensor core, TMEM)
 //     P  = exp2(S * scale * log2e - lse2)            dS = P * (dP - delta) * scale     (softmax warps, thread = q row)
-//     dV += P^T dO     dK += dS^T Q      (tensor core, accumulate in TMEM over the whole walk - no atomics, GQA summed)
+//     dV += P^T dO     dK += dS^T Q      (tensor core, accumulate in TMEM over the whole walk, GQA summed)
 //     dQ_partial = dS K                  (tensor core, into the TMEM columns dP has just left) -> tiled fp32 TMA reduction into dQ
 // A step's products run under the computations of the P / dS warps: dP under P, dV and the next step's S under dS, dQ and dK
 // under the next P. For that P and dS share one buffer (each waits for the products that read the other), which makes room for
@@ -21,13 +21,17 @@
 //   warps 4-11  softmax / dS (thread = q row; warps 4-7 take KV columns 0-63, warps 8-11 columns 64-127): P from S, then dS
 //               from dP, written as bf16 into 128-byte-swizzled shared memory; the same [q][kv] tiles serve as K-major A
 //               (dS for dQ) and as MN-major A (P^T, dS^T)
-//   warps 12-15 dQ drain (thread = q row), and at the end dV, dK (added where several CTAs share a tile, see fa_bwd_splits)
+//   warps 12-15 dQ drain (thread = q row), and at the end dV, dK (see share_sums where several CTAs share a tile)
+// dK and dV are the same bits on every call; dQ is added up in the order in which the KV tiles get there.
 // K_j ([kv][d]) is the K-major B operand of S and the MN-major B operand of dQ; Q_i and dO_i are K-major A operands of
 // S / dP and MN-major B operands of dK / dV: every tile is loaded once and read through two descriptors.
 //
 // Positions follow the forward kernel's segment description, so causal masks in context-parallel (zigzag) layouts are
 // exact. Reference behaviour replaced: materialised fp32 scores and their softmax per ring step
 // (reference: reference/57_ring_attention_backward_dp.py:39-69).
+#include <array>
+#include <type_traits>
+
 #include "pkb/api.h"
 #include "pkb/attention_api.h"
 #include "pkb/host.h"
@@ -55,7 +59,8 @@ struct FaBwdParams {
   int seg_scatter;
   float* dk_seg[16];
   float* dv_seg[16];
-  // splits > 1: that many CTAs share the walk of a KV tile and ADD their dK / dV to the zeroed buffers
+  // splits > 1: two clusters of splits / 2 CTAs share the walk of a KV tile. The dK / dV of a cluster meet in shared memory, the two
+  // clusters ADD theirs to the zeroed buffers (0 + a + b is the same in either order, so the result does not depend on timing).
   int splits;
   uint32_t* status;
   uint64_t budget_ns;
@@ -84,12 +89,16 @@ struct FbSmem {
   // dQ staging, 8 KiB per drain warp: two boxes of 32 rows x 32 fp32 columns (128-byte swizzle). A buffer of its own, so that
   // the reductions of step s run under the products and the P / dS computation of step s+1.
   static constexpr int kDqStage = kPDS + kPBytes;
+  // a shared tile's partial dV and dK, fp32, over the operand tiles of the finished walk; 16-byte accesses of 8 rows hit all banks
+  static constexpr int kPartPitch = D * 4 + 16;
+  static constexpr int kPartBytes = kFbTile * kPartPitch;
+  static_assert(2 * kPartBytes <= kPDS, "partial sums outgrew the operand tiles");
   static constexpr int kBars = kDqStage + 4 * 8192;
   static constexpr int kTotal = kBars + 320;
   static_assert(kTotal <= 232448, "shared-memory plan exceeds the 227 KiB a CTA may use");
 };
 
-// delta[b,h,s] = sum_d dO * O ; lse2 = lse * log2(e); dQ (and, where they are accumulated or not fully written, dK and dV) are
+// delta[b,h,s] = sum_d dO * O ; lse2 = lse * log2(e); dQ (and, where they are added to or not fully written, dK and dV) are
 // zero-filled on the way. Memory bound: D / 8 lanes per (head, position) with 16-byte accesses, positions fastest, so that
 // delta, lse and lse2 are runs of memory.
 template <int D>
@@ -179,7 +188,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int rep = d.hq / d.hkv;
-  // x: (batch, KV head, split), y: KV tile. x runs fastest, so the heavy tiles of all heads are started before any light one.
+  // x: (batch, KV head, split), y: KV tile. x runs fastest, so the heavy tiles of all heads are started before any light one. The
+  // first and the second half of a tile's splits are a cluster each.
   const int split = blockIdx.x % p.splits;
   const int kv_head = (blockIdx.x / p.splits) % d.hkv;
   const int batch = blockIdx.x / (p.splits * d.hkv);
@@ -286,6 +296,53 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       w.k = 0;
       ++w.head;
     }
+  };
+
+  // Sums of a shared tile: each CTA of the cluster holds the dV and dK of its part of the walk in shared memory, adds up its share of
+  // the rows over the CTAs in the order of their ranks and adds the sum to the result. Every thread of the cluster meets at the two
+  // barriers, whatever it waited for in vain before; `t`, `threads`: the threads that add.
+  const int csize = p.splits > 1 ? p.splits >> 1 : 1;
+  auto share_sums = [&](int t, int threads) {
+    cluster_sync_all();                  // every CTA's partial sums are in its shared memory
+    constexpr int kPerRow = D / 4;
+    const int rank = split % csize;
+    uint32_t has = 0;                    // ranks whose part of the walk is not empty
+    for (int c = 0; c < csize; ++c) {
+      const long long total = (long long)n_active * rep, first = split - rank + c;
+      if (total * (first + 1) / p.splits > total * first / p.splits) has |= 1u << c;
+    }
+    const int i_begin = 2 * kv_valid * kPerRow * rank / csize, i_end = 2 * kv_valid * kPerRow * (rank + 1) / csize;
+    // ITEMS x RANKS loads of a thread are in flight together
+    auto add_up = [&](auto items, auto ranks) {
+      constexpr int ITEMS = decltype(items)::value, RANKS = decltype(ranks)::value;
+      for (int i0 = i_begin + t; i0 < i_end; i0 += ITEMS * threads) {
+        float4 part[ITEMS][RANKS];
+#pragma unroll
+        for (int u = 0; u < ITEMS; ++u) {
+          const int i = i0 + u * threads, row2 = i / kPerRow;
+          const uint32_t src = sb + (row2 >= kv_valid ? S::kPartBytes + (row2 - kv_valid) * S::kPartPitch : row2 * S::kPartPitch) + (i % kPerRow) * 16;
+#pragma unroll
+          for (int c = 0; c < RANKS; ++c)
+            part[u][c] = i < i_end && ((has >> c) & 1u) ? ld_shared_cluster_v4(mapa_shared(src, c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < ITEMS; ++u) {
+          const int i = i0 + u * threads, row2 = i / kPerRow;
+          if (i >= i_end) break;
+          float4 v = part[u][0];
+#pragma unroll
+          for (int c = 1; c < RANKS; ++c) { v.x += part[u][c].x; v.y += part[u][c].y; v.z += part[u][c].z; v.w += part[u][c].w; }
+          const bool is_dk = row2 >= kv_valid;
+          red_add_v4_f32((is_dk ? p.dk : p.dv) + ((static_cast<long long>(kv_tok0) + (is_dk ? row2 - kv_valid : row2)) * d.hkv + kv_head) * D + (i % kPerRow) * 4,
+                         v.x, v.y, v.z, v.w);
+        }
+      }
+    };
+    if (has != 0) {
+      if (csize <= 4) add_up(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{});
+      else add_up(std::integral_constant<int, 2>{}, std::integral_constant<int, 8>{});
+    }
+    cluster_sync_all();                  // nobody's shared memory goes away while a peer still reads it
   };
 
   // `work`: false when no query sees this tile (warps 12-15 then store zeros into its dK / dV rows)
@@ -408,6 +465,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       else if (lane == 0) record_status(p.status, kStatusMbarTimeout, 650, 0, 0, 20, 0);
     }
     __syncwarp();
+    }
+    if (csize > 1) {                     // the two barriers of share_sums
+      cluster_sync_all();
+      cluster_sync_all();
     }
   } else if (warp < 12) {
     warpgroup_reg_inc<kFbRegsSoftmax>();
@@ -539,6 +600,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       if constexpr (TRACE) { if (warp == 4 && lane == 0) fb_trace(p, 1, 4, step); }
     }
     if (!ok && work && lane == 0) record_status(p.status, kStatusMbarTimeout, 650, 0, 0, 30, 0);
+    __syncwarp();
+    if (csize > 1) share_sums(threadIdx.x - 128, 384);
   } else {
     // ------------------------------ dQ drain, then dV / dK (thread = row) ------------------------------
     warpgroup_reg_inc<kFbRegsDrain>();
@@ -617,6 +680,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         dvp = p.dv_seg[kv_seg] + off;
         dkp = p.dk_seg[kv_seg] + off;
       }
+      const uint32_t part = sb + static_cast<uint32_t>(row) * S::kPartPitch;
 #pragma unroll
       for (int c = 0; c < DH / 32; ++c) {
         uint32_t rv[32], rk[32];
@@ -628,7 +692,19 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 32; ++i) { rv[i] = 0u; rk[i] = 0u; }
         }
-        if (row_ok && add) {
+        if (csize > 1) {                 // for share_sums: the products that read the operand tiles are complete
+          if (n_steps > 0) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(part + (c * 32 + i) * 4), "r"(rv[i]), "r"(rv[i + 1]), "r"(rv[i + 2]),
+                           "r"(rv[i + 3])
+                           : "memory");
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(part + S::kPartBytes + (c * 32 + i) * 4), "r"(rk[i]), "r"(rk[i + 1]),
+                           "r"(rk[i + 2]), "r"(rk[i + 3])
+                           : "memory");
+            }
+          }
+        } else if (row_ok && add) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             red_add_v4_f32(dvp + c * 32 + i, __uint_as_float(rv[i]), __uint_as_float(rv[i + 1]), __uint_as_float(rv[i + 2]),
@@ -649,6 +725,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     } else if (lane == 0 && !bad) {
       record_status(p.status, kStatusMbarTimeout, 650, 0, 0, 40, 0);
     }
+    __syncwarp();
+    if (csize > 1) share_sums(threadIdx.x - 128, 384);
   }
 
   tc_fence_before_sync();
@@ -664,11 +742,42 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   }
 }
 
+// Clusters of `ctas` CTAs of the backward kernel that fit the GPU at once (8 CTAs: 15 clusters, 4: 33, 3: 45, 2: 74 - a cluster stays
+// inside a group of 16 to 20 SMs).
+template <int D>
+static int fa_bwd_resident(int ctas) {
+  static const std::array<int, 9> table = [] {
+    std::array<int, 9> t{};
+    (void)cudaFuncSetAttribute(fa_bwd_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSmem<D>::kTotal);
+    for (int c = 1; c <= 8; ++c) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)c);
+      cfg.blockDim = dim3(kFbThreads);
+      cfg.dynamicSmemBytes = FbSmem<D>::kTotal;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)c;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&t[c], fa_bwd_kernel<D, false>, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        t[c] = c <= 2 ? sm_count() / c : 0;
+      }
+    }
+    return t;
+  }();
+  return table[ctas];
+}
+
 // CTAs per KV tile and head: as many as bring the longest walk (the first KV tile under a causal mask) down to an SM's share of all
 // steps; at least two steps each, eight where that makes more CTAs than SMs (a CTA's K and V loads and its dK / dV cost about one
-// and a half steps). With more than one, dK / dV are added up with fp32 reductions (in no fixed order, as dQ always is).
-// d = 128, causal: batch 2, S = 1024, 8 / 2 heads (32 tiles) 128 us on one CTA each, 39 us on four, 43 on eight; S = 4096, 16 / 4
-// heads (128 tiles) 334 us on one, 191 on two.
+// and a half steps). They are two clusters of at most 8; where all CTAs would fit the SMs, the clusters are made small enough that
+// they do so too. d = 128, us on 1 / 2 / 4 / 6 / 8 CTAs per tile: batch 2, S = 1024, 8 / 2 heads, causal (32 tiles) 128 / 66 / 48 / 58 / 58;
+// S = 1024, 2 / 1 heads, causal (8 tiles) 87 / 40 / 32 / 30 / 30; S = 1200, 8 / 1 heads, no mask (10 tiles) - / 164 / 95 / 73 / 60 and 52 on
+// 12; S = 4096, 16 / 4 heads, causal (128 tiles) 334 / 190. What the fixed order costs: 46 and 44 us for the first and the third
+// when every CTA added its sums to memory as it came.
+template <int D>
 static int fa_bwd_splits(const pkb_attn_desc& d, int kv_tiles) {
   const long long rep = d.hq / d.hkv;
   const long long rows_per_seg = d.num_q_segs == 1 ? d.sq : d.q_seg_rows;
@@ -690,7 +799,11 @@ static int fa_bwd_splits(const pkb_attn_desc& d, int kv_tiles) {
   const long long most = longest * rep;
   if (s * kv_tiles * heads > sms && s > most / 8) s = most / 8 > sms / (kv_tiles * heads) ? most / 8 : sms / (kv_tiles * heads);
   if (s > most / 2) s = most / 2;
-  return s < 1 ? 1 : (int)s;
+  if (s < 2) return 1;
+  int cluster = s < 16 ? (int)s / 2 : 8;
+  if (2 * cluster * kv_tiles * heads <= sms)
+    while (cluster > 1 && 2 * kv_tiles * heads > fa_bwd_resident<D>(cluster)) --cluster;
+  return 2 * cluster;
 }
 
 // KV rows of the buffer that lie in a segment (segments may overlap, so their lengths do not add up to it).
@@ -731,7 +844,7 @@ static int launch_fa_bwd(const pkb_attn_desc& d, const void* q, const void* k, c
   int kv_tiles = 0;
   for (int s = 0; s < d.num_kv_segs; ++s) kv_tiles += (d.kv_seg_len[s] + kFbTile - 1) / kFbTile;
   const bool scatter = dk_seg != nullptr && dv_seg != nullptr;
-  const int splits = scatter ? 1 : fa_bwd_splits(d, kv_tiles);
+  const int splits = scatter ? 1 : fa_bwd_splits<D>(d, kv_tiles);
   // every row of dK / dV is written by the main kernel unless rows lie outside all segments or CTAs add to them
   const long long kv_elems = !scatter && (splits > 1 || fa_bwd_covered(d) < d.skv) ? (long long)d.batch * d.skv * d.hkv * D : 0;
   CUtensorMap tdq;
@@ -766,9 +879,19 @@ static int launch_fa_bwd(const pkb_attn_desc& d, const void* q, const void* k, c
   constexpr int smem = FbSmem<D>::kTotal;
   PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   if (kv_tiles == 0) return kApiOk;
-  dim3 grid(d.hkv * d.batch * splits, kv_tiles);
-  kern<<<grid, kFbThreads, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
-  PKB_CHECK_CUDA(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(d.hkv * d.batch * splits), (unsigned)kv_tiles);
+  cfg.blockDim = dim3(kFbThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)splits / 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 2 ? 1 : 0;
+  PKB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tdo, tdq, p));
   return kApiOk;
 }
 

@@ -255,7 +255,8 @@ def flash_attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch
     ``dk_out`` / ``dv_out``: optional fp32 tensors shaped like k / v that receive the result;
     a caller that reduces them over ranks passes symmetric-heap tensors so that the collective needs no staging copy.
     Returns fp32 ``(dq, dk, dv)`` shaped like q, k, v. bf16 inputs with head dimension 64 or 128 run on the tcgen05
-    kernel (dK/dV accumulate in TMEM, dQ by fp32 vector reductions); anything else takes the PyTorch restatement."""
+    kernel (dK / dV accumulate in TMEM and repeat bit for bit; dQ is summed by fp32 TMA reductions in no fixed order); anything
+    else takes the PyTorch restatement."""
     D = q.shape[-1]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     squeeze = q.dim() == 3

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
                                                       (1, 2000, 129, 6, 3, 64, False), (1, 100, 900, 1, 1, 64, True), (1, 300, 2000, 16, 16, 128, True),
                                                       (4, 257, 257, 16, 8, 128, True)])
 def test_attention_backward_shared_between_ctas(B, sq, skv, hq, hkv, D, causal):
-    """dK / dV are then added up in global memory, so stale values in the buffers would show: they are filled with NaN first."""
+    """Every row of dK / dV is written by one CTA or another: stale values in the buffers would show, they are filled with NaN first."""
     from parallelkernelbench_b200.ops.attention import flash_attn_bwd, flash_attn_fwd
     from parallelkernelbench_b200.refs.attention import attention_bwd_positions_ref
 
@@ -65,3 +65,20 @@ def test_attention_backward_zeroes_uncovered_rows_beside_overlapping_segments():
     _, dk, dv = flash_attn_bwd(q, k, v, out, lse, dout, causal=False, kv_segments=[(C, 0, 2 * C), (C, 0, 2 * C)], dk_out=bufs[0], dv_out=bufs[1])
     for g in (dk, dv):
         assert (g[:, :C] == 0).all() and torch.isfinite(g).all() and (g[:, C:] != 0).any()
+
+
+# walks shared by two, four and eight CTAs; tiles whose walk is shorter than the cluster; a last tile with few rows
+@pytest.mark.parametrize("B,S,hq,hkv,D,causal", [(2, 1024, 8, 2, 128, True), (1, 1024, 2, 1, 128, True), (1, 700, 16, 4, 128, False), (1, 1500, 4, 1, 64, True),
+                                                 (1, 1100, 8, 4, 64, True), (1, 129, 8, 1, 128, True)])
+def test_attention_backward_repeats_dk_and_dv_bit_for_bit(B, S, hq, hkv, D, causal):
+    """The partial sums of a shared tile are added in the order of the CTAs, not of their arrival. (dQ is summed in no fixed order.)"""
+    from parallelkernelbench_b200.ops.attention import flash_attn_bwd, flash_attn_fwd
+
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, dout = (torch.randn(B, S, hq, D, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(B, S, hkv, D, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    out, lse = flash_attn_fwd(q, k, v, causal=causal)
+    _, dk, dv = flash_attn_bwd(q, k, v, out, lse, dout, causal=causal)
+    for _ in range(12):
+        _, dk2, dv2 = flash_attn_bwd(q, k, v, out, lse, dout, causal=causal)
+        assert torch.equal(dk, dk2) and torch.equal(dv, dv2)

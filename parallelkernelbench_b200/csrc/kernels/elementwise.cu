@@ -228,7 +228,7 @@ ce_stats_kernel(const T* __restrict__ logits, const long long* __restrict__ targ
   constexpr int kUnroll = 4;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const T* lr = logits + (long long)row * vocab_local;
-    float m = -INFINITY, sum = 0.f;
+    float m = -INFINITY, sum = 0.f, off = 0.f;
     for (int base = threadIdx.x * kPer; base < vocab_local; base += kCeThreads * kPer * kUnroll) {
       float f[kUnroll * kPer];
 #pragma unroll
@@ -256,14 +256,17 @@ ce_stats_kernel(const T* __restrict__ logits, const long long* __restrict__ targ
       float lm = f[0];
 #pragma unroll
       for (int j = 1; j < kUnroll * kPer; ++j) lm = fmaxf(lm, f[j]);
+      // off = -m * log2(e), rounded. All terms share its rounding (2e-5 of them at m = 400), which is undone at the end.
       if (lm > m) {
-        sum *= fast_exp2((m - lm) * kLog2eCe);     // m = -inf at first: 0 * 0
+        const float next = -lm * kLog2eCe;
+        if (m != -INFINITY) sum *= fast_exp2(next - off);
         m = lm;
+        off = next;
       }
-      const float off = m == -INFINITY ? 0.f : -m * kLog2eCe;
 #pragma unroll
       for (int j = 0; j < kUnroll * kPer; ++j) sum += fast_exp2(fmaf(f[j], kLog2eCe, off));
     }
+    if (m != -INFINITY) sum *= fast_exp2(fmaf(-m, kLog2eCe, -off));
     const float wm = warp_max(m);
     sum = warp_sum(wm == -INFINITY ? sum : sum * fast_exp2((m - wm) * kLog2eCe));
     const int warp = threadIdx.x >> 5;

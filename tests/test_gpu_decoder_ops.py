@@ -25,11 +25,28 @@ def test_ce_stats_edges(vocab, dtype):
     xd = x.double()
     assert torch.equal(st[:, 0], xd.max(-1).values)
     ref = torch.exp(xd - xd.max(-1, keepdim=True).values).sum(-1)
-    # ex2.approx is within 2 ulp, its argument within |x| * 2^-23 of exact, and the terms add up in fp32 over a few hundred per thread
-    torch.testing.assert_close(st[:, 1], ref, rtol=5e-5, atol=0)
+    # ex2.approx is within 2 ulp (2^-22), its argument d within |d| * 2^-23 of exact for a term exp(d) <= 1; a thread adds up to 98
+    # terms in fp32 (half an ulp each), then the lanes and warps another 21
+    torch.testing.assert_close(st[:, 1], ref, rtol=1e-5, atol=0)
     inside = ((tgt - 7) >= 0) & ((tgt - 7) < vocab)
     want = torch.where(inside, xd.gather(1, (tgt - 7).clamp(0, vocab - 1)[:, None])[:, 0], torch.zeros(rows, device="cuda", dtype=torch.float64))
     assert torch.equal(st[:, 2], want)
+
+
+@pytest.mark.parametrize("vocab,dtype", [(1001, torch.float32), (4096, torch.float32), (4096, torch.bfloat16)])
+def test_ce_stats_of_large_logits(vocab, dtype):
+    """Large maxima: the exponent is the difference from the maximum, whose rounding must not scale with the maximum itself."""
+    from parallelkernelbench_b200.ops import ce_local_stats
+
+    top = torch.tensor([80.3, 300.7, 400.9, 511.3, 777.1, -650.9], device="cuda")
+    x = torch.randn(6, vocab, device="cuda", generator=_gen(3)) + top[:, None] - 4
+    x[::2] -= 200                                        # every other row: one peak, the rest far below it
+    x[:, 17] = top + 4
+    x = x.to(dtype)
+    st = ce_local_stats(x, torch.zeros(6, dtype=torch.int64, device="cuda"), 0).double()
+    ref = torch.exp(x.double() - x.double().max(-1, keepdim=True).values).sum(-1)
+    # 2^-22 of the exponential, |d| exp(d) 2^-23 of its argument, half an ulp for each of at most 32 + 21 additions
+    torch.testing.assert_close(st[:, 1], ref, rtol=4e-6, atol=0)
 
 
 # columns: one load, the end of a block's 8192 columns, one load more

@@ -214,26 +214,29 @@ adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
 // ================================================================================================
 // Memory bound: the logits are read once. A thread keeps a running maximum and a running sum relative to it (rescaled when the
 // maximum moves, once per four 16-byte loads at most), so one pass gives both; four loads are in flight per thread. 4096 x 128256
-// bf16 (1.05 GB, 160 us at the copy bandwidth): 2044 us with two passes of 2-byte loads, 226 us now. The scalar form takes rows
-// whose length or address is not a multiple of 16 bytes.
-constexpr int kCeThreads = 512;
+// bf16 (1.05 GB, 160 us at the copy bandwidth): 1843 us with two passes of 2-byte loads, 202 us now. The scalar form takes rows
+// whose length or address is not a multiple of 16 bytes. ROW_THREADS: 512 (the block), or 32 for short rows, where most of a block's
+// threads would find nothing to load (see pkb_ce_stats).
+constexpr int kCeThreads = 512, kCeWarpFormThreads = 128, kCeUnroll = 4;
 constexpr float kLog2eCe = 1.4426950408889634f;
 
-template <typename T, bool VEC>
-__global__ void __launch_bounds__(kCeThreads)
+template <typename T, bool VEC, int ROW_THREADS>
+__global__ void __launch_bounds__(ROW_THREADS == 32 ? kCeWarpFormThreads : ROW_THREADS)
 ce_stats_kernel(const T* __restrict__ logits, const long long* __restrict__ target, float* __restrict__ stats, int rows,
                 int vocab_local, long long vocab_start) {
   __shared__ float red_m[kCeThreads / 32], red_s[kCeThreads / 32];
   constexpr int kPer = VEC ? 16 / (int)sizeof(T) : 1;   // elements per load
-  constexpr int kUnroll = 4;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+  constexpr int kUnroll = kCeUnroll;
+  constexpr bool kWarpRow = ROW_THREADS == 32;
+  constexpr int kRows = kWarpRow ? kCeWarpFormThreads / 32 : 1;   // rows a block works on at a time
+  for (int row = blockIdx.x * kRows + (kWarpRow ? (int)threadIdx.x >> 5 : 0); row < rows; row += gridDim.x * kRows) {
     const T* lr = logits + (long long)row * vocab_local;
     float m = -INFINITY, sum = 0.f, off = 0.f;
-    for (int base = threadIdx.x * kPer; base < vocab_local; base += kCeThreads * kPer * kUnroll) {
+    for (int base = (threadIdx.x & (ROW_THREADS - 1)) * kPer; base < vocab_local; base += ROW_THREADS * kPer * kUnroll) {
       float f[kUnroll * kPer];
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
-        const int i = base + u * kCeThreads * kPer;
+        const int i = base + u * ROW_THREADS * kPer;
         if (i < vocab_local) {
           if constexpr (!VEC) {
             f[u] = (float)lr[i];
@@ -264,25 +267,35 @@ ce_stats_kernel(const T* __restrict__ logits, const long long* __restrict__ targ
         off = next;
       }
 #pragma unroll
-      for (int j = 0; j < kUnroll * kPer; ++j) sum += fast_exp2(fmaf(f[j], kLog2eCe, off));
+      for (int j = 0; j < kUnroll * kPer; j += 2) {
+        float x0, x1;
+        fma2_bcast(x0, x1, f[j], f[j + 1], kLog2eCe, off);
+        sum += fast_exp2(x0);
+        sum += fast_exp2(x1);
+      }
     }
     if (m != -INFINITY) sum *= fast_exp2(fmaf(-m, kLog2eCe, -off));
     const float wm = warp_max(m);
     sum = warp_sum(wm == -INFINITY ? sum : sum * fast_exp2((m - wm) * kLog2eCe));
-    const int warp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) { red_m[warp] = wm; red_s[warp] = sum; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float mx = red_m[0];
-      for (int w = 1; w < kCeThreads / 32; ++w) mx = fmaxf(mx, red_m[w]);
-      float tot = 0.f;
-      for (int w = 0; w < kCeThreads / 32; ++w) tot += mx == -INFINITY ? red_s[w] : red_s[w] * fast_exp2((red_m[w] - mx) * kLog2eCe);
+    float mx = wm, tot = sum;
+    if constexpr (!kWarpRow) {
+      const int warp = threadIdx.x >> 5;
+      if ((threadIdx.x & 31) == 0) { red_m[warp] = wm; red_s[warp] = sum; }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        mx = red_m[0];
+        for (int w = 1; w < kCeThreads / 32; ++w) mx = fmaxf(mx, red_m[w]);
+        tot = 0.f;
+        for (int w = 0; w < kCeThreads / 32; ++w) tot += mx == -INFINITY ? red_s[w] : red_s[w] * fast_exp2((red_m[w] - mx) * kLog2eCe);
+      }
+    }
+    if ((threadIdx.x & (ROW_THREADS - 1)) == 0) {
       const long long t = target[row] - vocab_start;
       stats[(long long)row * 3 + 0] = mx;
       stats[(long long)row * 3 + 1] = tot;
       stats[(long long)row * 3 + 2] = (t >= 0 && t < vocab_local) ? (float)lr[t] : 0.f;
     }
-    __syncthreads();
+    if constexpr (!kWarpRow) __syncthreads();
   }
 }
 
@@ -503,17 +516,27 @@ int pkb_ce_stats(const void* logits, const void* target, void* stats, int rows, 
                  long long vocab_start, int dtype, void* stream) {
   if (rows == 0) return kApiOk;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int grid = rows < 148 * 8 ? rows : 148 * 8;
   const int per = dtype == 0 ? 8 : 4;
   const bool vec = vocab_local % per == 0 && ((uintptr_t)logits & 15) == 0;
-#define PKB_CE(T, V)                                                                                                          \
-  ce_stats_kernel<T, V><<<grid, kCeThreads, 0, s>>>(static_cast<const T*>(logits), static_cast<const long long*>(target),      \
-                                                    static_cast<float*>(stats), rows, vocab_local, vocab_start)
+  // A warp per row up to two of its passes (2048 bf16 elements), and up to eight where the rows fill the GPU. Us, warp / block per
+  // row: 8192 x 64 10.2 / 51.2, 8192 x 1000 12.3 / 55.3, 64 x 2048 8.2 / 8.1, 4096 x 8192 20.5 / 45.1; scalar form 8192 x 1001 16.2 / 30.7,
+  // 1024 x 4001 20.5 / 12.2.
+  const int pass = 32 * kCeUnroll * (vec ? per : 1);
+  const bool warp_row = vocab_local <= 2 * pass || (vocab_local <= 8 * pass && rows >= 16 * sm_count());
+  const int blocks = warp_row ? (rows + kCeWarpFormThreads / 32 - 1) / (kCeWarpFormThreads / 32) : rows;
+  const int grid = blocks < 148 * 8 ? blocks : 148 * 8;
+#define PKB_CE2(T, V, R)                                                                                                       \
+  ce_stats_kernel<T, V, R><<<grid, R == 32 ? kCeWarpFormThreads : R, 0, s>>>(static_cast<const T*>(logits),                      \
+                                                                           static_cast<const long long*>(target),              \
+                                                                           static_cast<float*>(stats), rows, vocab_local, vocab_start)
+#define PKB_CE(T, V) \
+  if (warp_row) PKB_CE2(T, V, 32); else PKB_CE2(T, V, kCeThreads)
   if (dtype == 0) {
-    if (vec) PKB_CE(__nv_bfloat16, true); else PKB_CE(__nv_bfloat16, false);
+    if (vec) { PKB_CE(__nv_bfloat16, true); } else { PKB_CE(__nv_bfloat16, false); }
   } else {
-    if (vec) PKB_CE(float, true); else PKB_CE(float, false);
+    if (vec) { PKB_CE(float, true); } else { PKB_CE(float, false); }
   }
+#undef PKB_CE2
 #undef PKB_CE
   PKB_CHECK_CUDA(cudaGetLastError());
   return kApiOk;

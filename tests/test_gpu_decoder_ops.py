@@ -33,6 +33,27 @@ def test_ce_stats_edges(vocab, dtype):
     assert torch.equal(st[:, 2], want)
 
 
+# a warp per row: up to two of its passes (bf16 2048, fp32 1024, scalar 256 elements) at any number of rows, up to eight where the rows
+# fill the GPU; one element more; more rows than the grid takes at a time
+@pytest.mark.parametrize("rows,vocab,dtype", [(7, 2048, torch.bfloat16), (7, 2056, torch.bfloat16), (2400, 8192, torch.bfloat16), (2400, 8200, torch.bfloat16),
+                                              (5, 1024, torch.float32), (2400, 4096, torch.float32), (2400, 1023, torch.bfloat16), (2400, 1025, torch.bfloat16),
+                                              (3, 255, torch.float32), (9999, 24, torch.bfloat16)])
+def test_ce_stats_of_short_rows(rows, vocab, dtype):
+    from parallelkernelbench_b200.ops import ce_local_stats
+
+    x = (torch.randn(rows, vocab, device="cuda", generator=_gen(rows)) * 5).to(dtype)
+    x[1] = float("-inf")
+    x[2, :-1] = float("-inf")
+    tgt = torch.randint(0, vocab, (rows,), device="cuda", generator=_gen(1))
+    st = ce_local_stats(x, tgt, 0).double()
+    xd = x.double()
+    mx = xd.max(-1).values
+    assert torch.equal(st[:, 0], mx) and torch.equal(st[:, 2], xd.gather(1, tgt[:, None])[:, 0])
+    ref = torch.exp(xd - mx[:, None].clamp(min=-1e30)).sum(-1)
+    # as above, with up to 256 terms per thread (half an ulp each, and they do not all fall to the same side)
+    torch.testing.assert_close(st[:, 1], ref, rtol=1e-5, atol=0)
+
+
 @pytest.mark.parametrize("vocab,dtype", [(1001, torch.float32), (4096, torch.float32), (4096, torch.bfloat16)])
 def test_ce_stats_of_large_logits(vocab, dtype):
     """Large maxima: the exponent is the difference from the maximum, whose rounding must not scale with the maximum itself."""

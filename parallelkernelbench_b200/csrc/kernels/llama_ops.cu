@@ -236,8 +236,22 @@ rmsnorm_bwd_scalar_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 // d logits of the mean cross-entropy over a vocabulary shard: (exp(logit - lse) - [col == target - vocab_start]) * scale,
 // written as bf16 in one pass (lse is the GLOBAL log-sum-exp of the row, natural log).
 // A block takes 8192 columns of one row at a time, four 16-byte loads in flight per thread, and the row's constants are read once
-// per block instead of once per 16 bytes. 4096 x 128256 (2.1 GB, 321 us at the copy bandwidth): 466 us before, 421 us now.
+// per block instead of once per 16 bytes. 4096 x 128256 (2.1 GB, 321 us at the copy bandwidth): 332 us, 415 us with the form below.
 constexpr int kCeBwdCols = 256 * 8 * 4;
+
+// Eight columns; t: the target's column relative to the first of them.
+__device__ __forceinline__ U4 ce_bwd8(const U4& v, float l, long long t, float scale) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = unpack_bf16x2(w[j]);
+    const float a = (__expf(f.x - l) - (t == 2 * j ? 1.f : 0.f)) * scale;
+    const float b = (__expf(f.y - l) - (t == 2 * j + 1 ? 1.f : 0.f)) * scale;
+    o[j] = pack_bf16x2(a, b);
+  }
+  return U4{o[0], o[1], o[2], o[3]};
+}
 
 __global__ void __launch_bounds__(256)
 ce_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const float* __restrict__ lse, const long long* __restrict__ target,
@@ -258,17 +272,24 @@ ce_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const float* __restrict_
     for (int u = 0; u < 4; ++u) {
       const int c = c_base + u * 2048;
       if (c >= V) break;
-      const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-      uint32_t o[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = unpack_bf16x2(w[j]);
-        const float a = (__expf(f.x - l) - ((long long)(c + 2 * j) == t ? 1.f : 0.f)) * scale;
-        const float b = (__expf(f.y - l) - ((long long)(c + 2 * j + 1) == t ? 1.f : 0.f)) * scale;
-        o[j] = pack_bf16x2(a, b);
-      }
-      st_global_v4(dst + c, U4{o[0], o[1], o[2], o[3]});
+      st_global_v4(dst + c, ce_bwd8(v[u], l, t - c, scale));
     }
+  }
+}
+
+// Rows of fewer than 8192 columns, which would leave threads of such a block without a load: 16 bytes per thread across row ends.
+// Us, this / the form above: 8192 x 64 6.7 / 22.6, 8192 x 1000 14.2 / 24.7, 4096 x 4096 20.5 / 22.6, 4096 x 8192 34.7 / 28.7.
+__global__ void __launch_bounds__(256)
+ce_bwd_short_kernel(const __nv_bfloat16* __restrict__ logits, const float* __restrict__ lse, const long long* __restrict__ target,
+                    __nv_bfloat16* __restrict__ dlog, long long rows, int V, long long vocab_start, float scale,
+                    const float* __restrict__ upstream) {
+  if (upstream != nullptr) scale *= *upstream;
+  const long long vec_per_row = V / 8;
+  const long long total = rows * vec_per_row;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / vec_per_row;
+    const int c = (int)(i - r * vec_per_row) * 8;
+    st_global_v4(dlog + r * V + c, ce_bwd8(ld_global_nc_v4(logits + r * V + c), lse[r], target[r] - vocab_start - c, scale));
   }
 }
 
@@ -506,10 +527,19 @@ extern "C" int pkb_ce_bwd(const void* logits, const void* lse, const void* targe
                           long long vocab_start, float scale, const void* upstream, void* stream) {
   PKB_CHECK_ARG(rows >= 0 && V > 0 && V % 8 == 0, "the vocabulary shard must be a positive multiple of 8");
   if (rows == 0) return kApiOk;
-  dim3 grid((V + kCeBwdCols - 1) / kCeBwdCols, rows < 32768 ? (unsigned)rows : 32768u);
-  ce_bwd_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(logits), static_cast<const float*>(lse), static_cast<const long long*>(target),
-      static_cast<__nv_bfloat16*>(dlog), rows, V, vocab_start, scale, static_cast<const float*>(upstream));
+  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(logits);
+  const float *lp = static_cast<const float*>(lse), *up = static_cast<const float*>(upstream);
+  const long long* tp = static_cast<const long long*>(target);
+  __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(dlog);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (V < kCeBwdCols) {
+    long long blocks = (rows * (V / 8) + 255) / 256;
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    ce_bwd_short_kernel<<<(int)blocks, 256, 0, s>>>(src, lp, tp, dst, rows, V, vocab_start, scale, up);
+  } else {
+    dim3 grid((V + kCeBwdCols - 1) / kCeBwdCols, rows < 32768 ? (unsigned)rows : 32768u);
+    ce_bwd_kernel<<<grid, 256, 0, s>>>(src, lp, tp, dst, rows, V, vocab_start, scale, up);
+  }
   PKB_CHECK_CUDA(cudaGetLastError());
   return kApiOk;
 }

@@ -71,7 +71,7 @@ def test_ce_stats_of_large_logits(vocab, dtype):
 
 
 # columns: one load, the end of a block's 8192 columns, one load more
-@pytest.mark.parametrize("rows,vocab", [(1, 8), (3, 8192), (3, 8200), (130, 1000)])
+@pytest.mark.parametrize("rows,vocab", [(1, 8), (3, 8192), (3, 8200), (130, 1000), (5, 8184), (3000, 64)])
 def test_ce_backward_edges(rows, vocab):
     from parallelkernelbench_b200.ops import ce_backward
 

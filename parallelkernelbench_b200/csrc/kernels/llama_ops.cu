@@ -179,7 +179,8 @@ rmsnorm_dgamma_kernel(const float* __restrict__ partial, int nblk, int H, float*
   }
 }
 
-// The form for hidden sizes that are not a multiple of 8 (2-byte accesses, one global atomic per block and column).
+// The form for hidden sizes that are not a multiple of 8 and for tensors off the 16-byte boundary (2-byte accesses, one global atomic
+// per block and column).
 template <int COLS_PER_THREAD>
 __global__ void __launch_bounds__(256)
 rmsnorm_bwd_scalar_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
@@ -575,7 +576,8 @@ extern "C" int pkb_rmsnorm_bwd_partials(int rows, int H) {
 
 // dx = gradient of the norm (+ res, bf16 [rows, H], may be null); the gain's gradient goes to dgamma (fp32 [H], may be null) and
 // dgamma_bf16 (may be null). partial: scratch of pkb_rmsnorm_bwd_partials(rows, H) x H fp32 values.
-// H % 8 != 0: res and dgamma_bf16 must be null and dgamma is accumulated into (zero-filled by the caller).
+// H % 8 != 0, or partial null (tensors off the 16-byte boundary): res and dgamma_bf16 must be null and dgamma is accumulated into
+// (zero-filled by the caller).
 extern "C" int pkb_rmsnorm_bwd(const void* x, const void* gamma, const void* dy, const void* res, void* dx, void* dgamma,
                                void* dgamma_bf16, void* partial, int rows, int H, float eps, void* stream) {
   PKB_CHECK_ARG(rows >= 0 && H > 0 && H <= 256 * 32, "hidden size must be at most 8192");
@@ -585,9 +587,9 @@ extern "C" int pkb_rmsnorm_bwd(const void* x, const void* gamma, const void* dy,
                       *dyp = static_cast<const __nv_bfloat16*>(dy), *rp = static_cast<const __nv_bfloat16*>(res);
   __nv_bfloat16* dxp = static_cast<__nv_bfloat16*>(dx);
   float* dgp = static_cast<float*>(dgamma);
-  if (H % 8 == 0) {
-    PKB_CHECK_ARG(partial != nullptr && (((uintptr_t)x | (uintptr_t)gamma | (uintptr_t)dy | (uintptr_t)res | (uintptr_t)dx | (uintptr_t)partial) & 15) == 0,
-                  "16-byte aligned tensors and a partial buffer are required");
+  if (H % 8 == 0 && partial != nullptr) {
+    PKB_CHECK_ARG((((uintptr_t)x | (uintptr_t)gamma | (uintptr_t)dy | (uintptr_t)res | (uintptr_t)dx | (uintptr_t)partial) & 15) == 0,
+                  "the partial buffer goes with 16-byte aligned tensors");
     const int blocks = pkb_rmsnorm_bwd_partials(rows, H);
     float* pp = static_cast<float*>(partial);
 #define PKB_RMSB(CH)                                                                                          \

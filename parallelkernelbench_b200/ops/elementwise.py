@@ -169,7 +169,8 @@ def rmsnorm_bwd(x: torch.Tensor, gamma: torch.Tensor, dy: torch.Tensor, eps: flo
     xc, dyc, gc = x.contiguous(), dy.contiguous(), gamma.reshape(-1).contiguous()
     dx = torch.empty_like(xc)
     lib = nv.cuda_lib()
-    nblk = lib.pkb_rmsnorm_bwd_partials(rows, H)
+    aligned = (xc.data_ptr() | gc.data_ptr() | dyc.data_ptr()) % 16 == 0          # contiguous views may start anywhere
+    nblk = lib.pkb_rmsnorm_bwd_partials(rows, H) if aligned else 0
     dg = torch.empty(H, dtype=torch.float32, device=x.device) if nblk else torch.zeros(H, dtype=torch.float32, device=x.device)
     part = torch.empty((nblk, H), dtype=torch.float32, device=x.device) if nblk else None
     nv.check(lib.pkb_rmsnorm_bwd(nv.ptr(xc), nv.ptr(gc), nv.ptr(dyc), None, nv.ptr(dx), nv.ptr(dg), None, nv.ptr(part), rows, H,

@@ -102,6 +102,23 @@ def test_rmsnorm_backward_edges(rows, H):
     torch.testing.assert_close(dg.double(), gd.grad, rtol=1e-5, atol=1e-5 * rows ** 0.5 * 4)   # fp32 sums over the rows
 
 
+@pytest.mark.parametrize("moved", ["x", "dy", "gamma"])
+def test_rmsnorm_backward_of_tensors_off_the_16_byte_boundary(moved):
+    from parallelkernelbench_b200.ops import rmsnorm_bwd
+
+    rows, H = 37, 256
+    t = {"x": torch.randn(rows, H, device="cuda", generator=_gen(1)).to(torch.bfloat16), "dy": torch.randn(rows, H, device="cuda", generator=_gen(2)).to(torch.bfloat16),
+         "gamma": torch.randn(H, device="cuda", generator=_gen(3)).to(torch.bfloat16)}
+    dx, dg = rmsnorm_bwd(t["x"], t["gamma"], t["dy"], 1e-5)
+    off = torch.empty(t[moved].numel() + 1, device="cuda", dtype=torch.bfloat16)[1:].view(t[moved].shape).copy_(t[moved])
+    assert off.is_contiguous() and off.data_ptr() % 16 == 2
+    t[moved] = off
+    dx2, dg2 = rmsnorm_bwd(t["x"], t["gamma"], t["dy"], 1e-5)
+    # fp32 sums in another order: one step of bf16, and the bound of the gain's gradient above
+    torch.testing.assert_close(dx2.float(), dx.float(), rtol=2 ** -7, atol=1e-5)
+    torch.testing.assert_close(dg2, dg, rtol=1e-5, atol=1e-5 * rows ** 0.5 * 4)
+
+
 # counts around the four elements of an access, more than one sweep of the grid, and tensors off the 16-byte boundary (scalar form)
 @pytest.mark.parametrize("n", [1, 3, 4, 7, 4099, 148 * 16 * 256 * 8 + 5])
 @pytest.mark.parametrize("offset", [0, 1])

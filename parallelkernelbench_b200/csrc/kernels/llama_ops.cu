@@ -61,20 +61,29 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __r
 // the reduction of the current one, so a block always has a row in flight. 4096 x 4096 (100 MB, 15 us at the copy bandwidth):
 // 49 us with 2-byte accesses and a global atomic per block and column, 21 us now and 5 us
 // for the partial rows.
+// ROW_WARPS: warps that share a row; a block of 8 holds 8 / ROW_WARPS rows at a time. With one
+// row per block the other threads of a short row had nothing to do: 16384 x 128 55.5 us, 19.2 now (2-byte form 38.8), 65536 x 64 175 / 31.7
+// (124), 4096 x 1024 25.6 / 19.5 (21.5), 2048 x 512 19.2 / 15.3 (16.6).
 constexpr int kRmsBwdBlocks = 148 * 2;
 
-template <int CH, bool RES>
+// Rows a block holds at a time.
+static int rmsnorm_bwd_rows_per_block(int H) { return H <= 256 ? 8 : H <= 512 ? 4 : H <= 1024 ? 2 : 1; }
+
+template <int CH, bool RES, int ROW_WARPS>
 __global__ void __launch_bounds__(256)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ dy,
                    const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int H,
-                   float eps) {
+                   float eps, float* __restrict__ dg32, __nv_bfloat16* __restrict__ dg16) {
+  constexpr int kRows = 8 / ROW_WARPS, kRowThreads = 32 * ROW_WARPS;
+  static_assert(CH == 1 || kRows == 1, "rows of more than one chunk have the block to themselves");
   __shared__ float red[2][2][8];
   float dg[CH][8];
   U4 gam[CH], xc[CH], dc[CH];
-  const int row0 = blockIdx.x;
+  const int slot = (int)threadIdx.x / kRowThreads, tx = (int)threadIdx.x & (kRowThreads - 1);
+  const int row0 = blockIdx.x * kRows + slot, step = gridDim.x * kRows;
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
-    const int i = (c * 256 + (int)threadIdx.x) * 8;
+    const int i = (c * kRowThreads + tx) * 8;
     gam[c] = xc[c] = dc[c] = U4{0u, 0u, 0u, 0u};
     if (i < H) {
       gam[c] = ld_global_nc_v4(gamma + i);
@@ -87,19 +96,19 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     for (int j = 0; j < 8; ++j) dg[c][j] = 0.f;
   }
   int par = 0;
-  for (int row = row0; row < rows; row += gridDim.x, par ^= 1) {
-    const int nrow = row + (int)gridDim.x;
+  for (int row = row0; row - slot < rows; row += step, par ^= 1) {     // all warps of a block take the same number of steps
+    const int nrow = row + step;
     U4 xn[CH], dn[CH], rv[RES ? CH : 1];
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-      const int i = (c * 256 + (int)threadIdx.x) * 8;
+      const int i = (c * kRowThreads + tx) * 8;
       xn[c] = dn[c] = U4{0u, 0u, 0u, 0u};
       if (i < H) {
         if (nrow < rows) {
           xn[c] = ld_global_nc_v4(x + (long long)nrow * H + i);
           dn[c] = ld_global_nc_v4(dy + (long long)nrow * H + i);
         }
-        if constexpr (RES) rv[c] = ld_global_nc_v4(res + (long long)row * H + i);
+        if constexpr (RES) rv[c] = row < rows ? ld_global_nc_v4(res + (long long)row * H + i) : U4{0u, 0u, 0u, 0u};
       }
     }
     float ss = 0.f, dot = 0.f;
@@ -116,16 +125,19 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     }
     ss = warp_sum(ss);
     dot = warp_sum(dot);
-    if ((threadIdx.x & 31) == 0) { red[par][0][threadIdx.x >> 5] = ss; red[par][1][threadIdx.x >> 5] = dot; }
-    __syncthreads();     // one per row: the next row writes the other half of red
-    float tss = 0.f, tdot = 0.f;
+    float tss = ss, tdot = dot;
+    if constexpr (ROW_WARPS > 1) {
+      if ((threadIdx.x & 31) == 0) { red[par][0][threadIdx.x >> 5] = ss; red[par][1][threadIdx.x >> 5] = dot; }
+      __syncthreads();     // one per row: the next row writes the other half of red
+      tss = tdot = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) { tss += red[par][0][w]; tdot += red[par][1][w]; }
+      for (int w = 0; w < ROW_WARPS; ++w) { tss += red[par][0][slot * ROW_WARPS + w]; tdot += red[par][1][slot * ROW_WARPS + w]; }
+    }
     const float rstd = rsqrtf(tss / (float)H + eps);
     const float mean_term = tdot * rstd / (float)H;      // mean(dxhat * xhat), xhat = x * rstd
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
-      const int i = (c * 256 + (int)threadIdx.x) * 8;
+      const int i = (c * kRowThreads + tx) * 8;
       const uint32_t xw[4] = {xc[c].x, xc[c].y, xc[c].z, xc[c].w}, dw[4] = {dc[c].x, dc[c].y, dc[c].z, dc[c].w},
                      gw[4] = {gam[c].x, gam[c].y, gam[c].z, gam[c].w};
       uint32_t o[4];
@@ -141,21 +153,51 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
           a1 += rf.y;
         }
         o[j] = pack_bf16x2(a0, a1);
-        dg[c][2 * j] += df.x * h0;
-        dg[c][2 * j + 1] += df.y * h1;
+        if (row < rows) {
+          dg[c][2 * j] += df.x * h0;
+          dg[c][2 * j + 1] += df.y * h1;
+        }
       }
-      if (i < H) st_global_v4(dx + (long long)row * H + i, U4{o[0], o[1], o[2], o[3]});
+      if (i < H && row < rows) st_global_v4(dx + (long long)row * H + i, U4{o[0], o[1], o[2], o[3]});
       xc[c] = xn[c];
       dc[c] = dn[c];
     }
   }
-#pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int i = (c * 256 + (int)threadIdx.x) * 8;
-    if (i < H) {
+  // a block by itself has the whole sum: no second launch
+  auto emit = [&](int i, const float* v) {
+    if (gridDim.x > 1) {
       float4* pr = reinterpret_cast<float4*>(partial + (long long)blockIdx.x * H + i);
-      pr[0] = make_float4(dg[c][0], dg[c][1], dg[c][2], dg[c][3]);
-      pr[1] = make_float4(dg[c][4], dg[c][5], dg[c][6], dg[c][7]);
+      pr[0] = make_float4(v[0], v[1], v[2], v[3]);
+      pr[1] = make_float4(v[4], v[5], v[6], v[7]);
+      return;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (dg32) dg32[i + j] = v[j];
+      if (dg16) dg16[i + j] = __float2bfloat16_rn(v[j]);
+    }
+  };
+  if constexpr (kRows == 1) {
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int i = (c * kRowThreads + tx) * 8;
+      if (i < H) emit(i, dg[c]);
+    }
+  } else {                 // the rows of the block, in order
+    __shared__ float4 sums[kRows - 1][kRowThreads * 2];
+    if (slot > 0) {
+      sums[slot - 1][tx] = make_float4(dg[0][0], dg[0][1], dg[0][2], dg[0][3]);
+      sums[slot - 1][kRowThreads + tx] = make_float4(dg[0][4], dg[0][5], dg[0][6], dg[0][7]);
+    }
+    __syncthreads();
+    if (slot == 0 && tx * 8 < H) {
+#pragma unroll
+      for (int r = 0; r < kRows - 1; ++r) {
+        const float4 a = sums[r][tx], b = sums[r][kRowThreads + tx];
+        dg[0][0] += a.x; dg[0][1] += a.y; dg[0][2] += a.z; dg[0][3] += a.w;
+        dg[0][4] += b.x; dg[0][5] += b.y; dg[0][6] += b.z; dg[0][7] += b.w;
+      }
+      emit(tx * 8, dg[0]);
     }
   }
 }
@@ -571,7 +613,9 @@ extern "C" int pkb_swiglu_bwd(const void* gu, const void* da, void* dgu, long lo
 // that take the scalar form.
 extern "C" int pkb_rmsnorm_bwd_partials(int rows, int H) {
   if (H % 8 != 0) return 0;
-  return rows < kRmsBwdBlocks ? rows : kRmsBwdBlocks;
+  const int per = rmsnorm_bwd_rows_per_block(H), blocks = (int)(((long long)rows + per - 1) / per);
+  if (blocks <= 4) return rows > 0 ? 1 : 0;      // a few steps of one block are shorter than the second launch
+  return blocks < kRmsBwdBlocks ? blocks : kRmsBwdBlocks;
 }
 
 // dx = gradient of the norm (+ res, bf16 [rows, H], may be null); the gain's gradient goes to dgamma (fp32 [H], may be null) and
@@ -592,14 +636,22 @@ extern "C" int pkb_rmsnorm_bwd(const void* x, const void* gamma, const void* dy,
                   "the partial buffer goes with 16-byte aligned tensors");
     const int blocks = pkb_rmsnorm_bwd_partials(rows, H);
     float* pp = static_cast<float*>(partial);
-#define PKB_RMSB(CH)                                                                                          \
-    {                                                                                                         \
-      if (rp) rmsnorm_bwd_kernel<CH, true><<<blocks, 256, 0, s>>>(xp, gp, dyp, rp, dxp, pp, rows, H, eps);     \
-      else rmsnorm_bwd_kernel<CH, false><<<blocks, 256, 0, s>>>(xp, gp, dyp, rp, dxp, pp, rows, H, eps);       \
+    __nv_bfloat16* dg16 = static_cast<__nv_bfloat16*>(dgamma_bf16);
+#define PKB_RMSB(CH, RW)                                                                                                       \
+    {                                                                                                                          \
+      if (rp) rmsnorm_bwd_kernel<CH, true, RW><<<blocks, 256, 0, s>>>(xp, gp, dyp, rp, dxp, pp, rows, H, eps, dgp, dg16);       \
+      else rmsnorm_bwd_kernel<CH, false, RW><<<blocks, 256, 0, s>>>(xp, gp, dyp, rp, dxp, pp, rows, H, eps, dgp, dg16);         \
     }
-    if (H <= 2048) PKB_RMSB(1) else if (H <= 4096) PKB_RMSB(2) else PKB_RMSB(4)
+    switch (rmsnorm_bwd_rows_per_block(H)) {
+      case 8: PKB_RMSB(1, 1) break;
+      case 4: PKB_RMSB(1, 2) break;
+      case 2: PKB_RMSB(1, 4) break;
+      default:
+        if (H <= 2048) PKB_RMSB(1, 8) else if (H <= 4096) PKB_RMSB(2, 8) else PKB_RMSB(4, 8)
+    }
 #undef PKB_RMSB
-    rmsnorm_dgamma_kernel<<<(H + 31) / 32, 256, 0, s>>>(pp, blocks, H, dgp, static_cast<__nv_bfloat16*>(dgamma_bf16));
+    if (blocks > 1)
+      rmsnorm_dgamma_kernel<<<(H + 31) / 32, 256, 0, s>>>(pp, blocks, H, dgp, dg16);
   } else {
     PKB_CHECK_ARG(res == nullptr && dgamma_bf16 == nullptr && dgamma != nullptr, "the scalar form has no residual and writes an fp32 gain gradient");
     const int blocks = rows < 148 * 4 ? rows : 148 * 4;

@@ -85,9 +85,10 @@ def test_ce_backward_edges(rows, vocab):
     torch.testing.assert_close(got.double(), ref * 0.5, rtol=2 ** -8, atol=1e-6)
 
 
-# hidden sizes at the edges of the one-, two- and four-chunk forms and the scalar form (no multiple of 8); rows below, at and
-# beyond one per block
-@pytest.mark.parametrize("rows,H", [(1, 8), (297, 2048), (296, 2056), (593, 4096), (40, 4104), (700, 8192), (33, 100)])
+# hidden sizes at the edges of the one-, two- and four-chunk forms, of the forms with several rows per block and of the scalar form
+# (no multiple of 8); rows below, at and beyond one step of the grid, and of a single block
+@pytest.mark.parametrize("rows,H", [(1, 8), (297, 2048), (296, 2056), (593, 4096), (40, 4104), (700, 8192), (33, 100), (2369, 256), (8, 256), (9, 248),
+                                    (1185, 512), (4, 264), (2000, 520), (593, 1024), (2, 1000), (3, 1032), (4, 8192), (5, 4096), (32, 64), (33, 64)])
 def test_rmsnorm_backward_edges(rows, H):
     from parallelkernelbench_b200.ops import rmsnorm_bwd
 

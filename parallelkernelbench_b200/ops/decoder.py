@@ -81,6 +81,7 @@ def embed_grad_fp8_supported(n: int, hidden: int) -> bool:
 def embed_grad_fp8(dx: torch.Tensor, tokens: torch.Tensor, vocab: int, hidden: int, padded: int):
     """Gradient of :func:`embed_fp8` in the wire format of the gradient exchange: e4m3 bytes [padded] and fp32 scales
     [padded / 128] of the dense [vocab, hidden] gradient (bf16-rounded sums over a token's positions; zero rows have scale 1)."""
+    dx = dx if dx.data_ptr() % 16 == 0 else dx.clone()
     q = torch.zeros(padded, dtype=torch.uint8, device=dx.device)
     s = torch.ones(padded // 128, dtype=torch.float32, device=dx.device)
     nv.check(_fn("pkb_embed_grad_fp8")(dx.data_ptr(), tokens.data_ptr(), tokens.numel(), vocab, hidden, q.data_ptr(), s.data_ptr(),

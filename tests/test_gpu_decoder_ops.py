@@ -182,8 +182,9 @@ def test_qkv_rope_split_and_merge(tokens, hq, hkv, d):
     torch.testing.assert_close(got.float(), want, rtol=2 ** -8, atol=1e-6)
 
 
-# repeated tokens (first, last and middle positions), more positions than one mask word, the two ends of the table
-@pytest.mark.parametrize("n,vocab,H", [(1, 5, 128), (33, 7, 256), (257, 1000, 640)])
+# repeated tokens (first, last and middle positions), more positions than one mask word and than 32 of them, tokens repeated less,
+# as often and more often than rows are in flight, the two ends of the table
+@pytest.mark.parametrize("n,vocab,H", [(1, 5, 128), (33, 7, 256), (257, 1000, 640), (257, 3, 2176), (16, 2, 128), (1100, 2, 256), (16384, 5000, 128)])
 def test_embedding_wire_format(n, vocab, H):
     from parallelkernelbench_b200.ops import fp8_dequantize_1x128, fp8_quantize_1x128
     from parallelkernelbench_b200.ops.decoder import embed_fp8, embed_grad_fp8
@@ -191,15 +192,18 @@ def test_embedding_wire_format(n, vocab, H):
     table = torch.randn(vocab, H, device="cuda", generator=_gen(1))
     q, s = fp8_quantize_1x128(table)
     tok = torch.randint(0, vocab, (n,), device="cuda", generator=_gen(2))
-    tok[0], tok[-1] = vocab - 1, vocab - 1 if n > 1 else vocab - 1
+    tok[0] = vocab - 1
+    if n > 2:
+        tok[1], tok[-1] = 0, vocab - 1 if n == 257 else 0
     x = embed_fp8(q.view(-1), s.view(-1), tok, vocab, H)
     assert torch.equal(x, fp8_dequantize_1x128(q, s)[tok])
     dx = torch.randn(n, H, device="cuda", generator=_gen(3)).to(torch.bfloat16)
     padded = vocab * H + 256
     gq, gs = embed_grad_fp8(dx, tok, vocab, H, padded)
-    dense = torch.zeros(vocab, H, device="cuda")
-    for i in range(n):                                    # fp32 sums in position order
-        dense[tok[i]] += dx[i].float()
+    dense = torch.zeros(vocab, H)
+    for i, row in zip(tok.tolist(), dx.float().cpu()):    # fp32 sums in position order
+        dense[i] += row
+    dense = dense.cuda()
     wq, ws = fp8_quantize_1x128(torch.nn.functional.pad(dense.to(torch.bfloat16).reshape(-1), (0, 256)).view(-1, 128))
     assert torch.equal(gq, wq.view(-1)) and torch.equal(gs, ws.view(-1))
 

@@ -463,10 +463,12 @@ add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __rest
 
 // Embedding lookup from the wire format: row `tokens[t]` of a [vocab, H] table held as e4m3 bytes with one fp32 scale per 128
 // consecutive elements, as bf16. Only the rows that are looked up are converted (the whole table is 1.6 GB of traffic at
-// 128256 x 4096, 245 us; 4096 rows of it are 50 MB).
+// 128256 x 4096, 245 us; 4096 rows of it are 50 MB). A token outside the table gives a zero row and a status word.
+constexpr uint32_t kEmbedKernelId = 910;
+
 __global__ void __launch_bounds__(256)
 embed_fp8_kernel(const uint8_t* __restrict__ table, const float* __restrict__ scales, const long long* __restrict__ tokens,
-                 __nv_bfloat16* __restrict__ out, int n_tokens, int vocab, int H) {
+                 __nv_bfloat16* __restrict__ out, int n_tokens, int vocab, int H, uint32_t* status) {
   const int per_row = H >> 4;
   const unsigned total = (unsigned)n_tokens * per_row;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -486,6 +488,8 @@ embed_fp8_kernel(const uint8_t* __restrict__ table, const float* __restrict__ sc
         o[2 * j] = pack_bf16x2(f0.x * sc, f0.y * sc);
         o[2 * j + 1] = pack_bf16x2(f1.x * sc, f1.y * sc);
       }
+    } else if (c == 0) {
+      record_status(status, kStatusBadArgument, kEmbedKernelId, 0, 0, 1, t);
     }
     st_global_v4(out + (long long)t * H + c, U4{o[0], o[1], o[2], o[3]});
     st_global_v4(out + (long long)t * H + c + 8, U4{o[4], o[5], o[6], o[7]});
@@ -505,13 +509,16 @@ constexpr int kEmbedGradThreads = 256;
 
 __global__ void __launch_bounds__(kEmbedGradThreads)
 embed_grad_fp8_kernel(const __nv_bfloat16* __restrict__ dx, const long long* __restrict__ tokens, int n_tokens, int vocab, int H,
-                      uint8_t* __restrict__ q, float* __restrict__ s) {
+                      uint8_t* __restrict__ q, float* __restrict__ s, uint32_t* status) {
   extern __shared__ uint32_t hits[];                   // one bit per other position that holds the same token
   __shared__ int s_earlier, s_count;
   constexpr int kWarps = kEmbedGradThreads / 32, kFlight = 8;
   const int t = blockIdx.x;
   const long long tok = tokens[t];
-  if (tok < 0 || tok >= vocab) return;
+  if (tok < 0 || tok >= vocab) {
+    if (threadIdx.x == 0) record_status(status, kStatusBadArgument, kEmbedKernelId, 0, 0, 2, t);
+    return;
+  }
   if (threadIdx.x == 0) s_earlier = s_count = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -764,7 +771,7 @@ extern "C" int pkb_embed_fp8(const void* table, const void* scales, const void* 
   if (blocks > 148 * 8) blocks = 148 * 8;
   embed_fp8_kernel<<<(int)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint8_t*>(table), static_cast<const float*>(scales), static_cast<const long long*>(tokens),
-      static_cast<__nv_bfloat16*>(out), n, vocab, H);
+      static_cast<__nv_bfloat16*>(out), n, vocab, H, status_block_device_ptr());
   PKB_CHECK_CUDA(cudaGetLastError());
   return kApiOk;
 }
@@ -780,7 +787,8 @@ extern "C" int pkb_embed_grad_fp8(const void* dx, const void* tokens, int n, int
   const int smem = (n + 31) / 32 * 4 + n * 2;          // at most 34 KiB
   embed_grad_fp8_kernel<<<n, kEmbedGradThreads, smem, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(dx),
                                                                          static_cast<const long long*>(tokens), n, vocab, H,
-                                                                         static_cast<uint8_t*>(q), static_cast<float*>(s));
+                                                                         static_cast<uint8_t*>(q), static_cast<float*>(s),
+                                                                         status_block_device_ptr());
   PKB_CHECK_CUDA(cudaGetLastError());
   return kApiOk;
 }

@@ -381,6 +381,10 @@ class FSDPLlama:
 
     # -- one training step -------------------------------------------------------------------------
     def step(self, tokens: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+        if self.impl == "ours":
+            from .. import _native as nv
+
+            nv.raise_on_status(sync=False)         # what an earlier step's kernels reported
         self.steps += 1
         return self._step_ours(tokens, targets) if self.impl == "ours" else self._step_torch(tokens, targets)
 
@@ -395,7 +399,8 @@ class FSDPLlama:
     @torch.no_grad()
     def _step_ours(self, tokens: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
         """Forward and backward in the order the data allows, without a tape: every layer is one native call each way, and a
-        group's gradient is exchanged and applied as soon as it exists."""
+        group's gradient is exchanged and applied as soon as it exists. A token outside the vocabulary is reported by the status
+        words, which the next step raises (or ``_native.raise_on_status`` before it)."""
         from ..ops import adam_step, ce_backward, ce_local_stats, gemm_bf16, gemm_bf16_kn, gemm_bf16_tn, rmsnorm, rmsnorm_bwd
         from ..ops.decoder import ce_loss, embed_fp8, embed_grad_fp8, embed_grad_fp8_supported
 

@@ -65,7 +65,8 @@ class DecoderLayer:
 
 
 def embed_fp8(table: torch.Tensor, scales: torch.Tensor, tokens: torch.Tensor, vocab: int, hidden: int) -> torch.Tensor:
-    """Rows ``tokens`` of an e4m3 table with 1x128 scales (flat buffers) as bf16 [n, hidden]; ``hidden % 16 == 0``."""
+    """Rows ``tokens`` of an e4m3 table with 1x128 scales (flat buffers) as bf16 [n, hidden]; ``hidden % 16 == 0``. A token
+    outside the table gives a zero row and records a status (``_native.raise_on_status``)."""
     n = tokens.numel()
     out = torch.empty((n, hidden), dtype=torch.bfloat16, device=table.device)
     nv.check(_fn("pkb_embed_fp8")(table.data_ptr(), scales.data_ptr(), tokens.data_ptr(), out.data_ptr(), n, vocab, hidden, nv.raw_stream(table)),

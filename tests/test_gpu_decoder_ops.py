@@ -208,6 +208,47 @@ def test_embedding_wire_format(n, vocab, H):
     assert torch.equal(gq, wq.view(-1)) and torch.equal(gs, ws.view(-1))
 
 
+@pytest.mark.parametrize("bad", [-1, 7, 1 << 40])
+def test_tokens_outside_the_table_are_reported(bad):
+    from parallelkernelbench_b200 import _native as nv
+    from parallelkernelbench_b200.ops import fp8_quantize_1x128
+    from parallelkernelbench_b200.ops.decoder import embed_fp8, embed_grad_fp8
+
+    vocab, H = 7, 256
+    q, s = fp8_quantize_1x128(torch.randn(vocab, H, device="cuda", generator=_gen(1)))
+    tok = torch.tensor([0, bad, 6], device="cuda")
+    x = embed_fp8(q.view(-1), s.view(-1), tok, vocab, H)
+    with pytest.raises(nv.KernelStatusError, match="BAD_ARGUMENT.*tile=1"):
+        nv.raise_on_status()
+    assert (x[1] == 0).all() and (x[0] != 0).any()
+    embed_grad_fp8(x, tok, vocab, H, vocab * H)
+    with pytest.raises(nv.KernelStatusError, match="BAD_ARGUMENT.*tile=1"):
+        nv.raise_on_status()
+
+
+def test_a_step_on_a_token_outside_the_vocabulary_is_reported():
+    from parallelkernelbench_b200 import _native as nv
+    from parallelkernelbench_b200.models.llama import FSDPLlama, LlamaConfig
+    from parallelkernelbench_b200.parallel import init_context
+
+    ctx = init_context()
+    try:
+        m = FSDPLlama(ctx, LlamaConfig(layers=1, hidden=256, ffn=256, heads=2, kv_heads=1, vocab=512, seq=64))
+        tok = torch.arange(64, device="cuda")
+        m.step(tok, tok)
+        m.step(tok, tok)
+        bad = tok.clone()
+        bad[9] = 512
+        m.step(bad, tok)
+        torch.cuda.synchronize()
+        with pytest.raises(nv.KernelStatusError, match="BAD_ARGUMENT"):
+            m.step(tok, tok)
+        assert m.steps == 3
+        m.step(tok, tok)
+    finally:
+        ctx.finalize()
+
+
 @pytest.mark.parametrize("rows,W", [(1, 1), (1025, 3)])
 def test_ce_loss_of_several_shards(rows, W):
     from parallelkernelbench_b200.ops.decoder import ce_loss

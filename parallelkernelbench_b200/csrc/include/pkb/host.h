@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <array>
 #include <string>
 
 namespace pkb {
@@ -63,5 +64,30 @@ int encode_tmap_3d(CUtensorMap* out, int dtype, const void* base, uint64_t inner
                    uint32_t box_inner, uint32_t box_mid, uint32_t box_outer, int swizzle);
 
 int sm_count();
+
+// [c] = clusters of c CTAs (1 to 8) of this kernel that fit the GPU at once. The kernel's shared-memory limit is raised on the way. For
+// rules on cluster sizes: keep it in a function-local static.
+template <typename Kernel>
+std::array<int, 9> resident_clusters(Kernel kern, int threads, int smem_bytes) {
+  std::array<int, 9> t{};
+  (void)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+  for (int c = 1; c <= 8; ++c) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)c);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem_bytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&t[c], kern, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      t[c] = 0;
+    }
+  }
+  return t;
+}
 
 }  // namespace pkb

@@ -742,34 +742,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   }
 }
 
-// Clusters of `ctas` CTAs of the backward kernel that fit the GPU at once (8 CTAs: 15 clusters, 4: 33, 3: 45, 2: 74 - a cluster stays
-// inside a group of 16 to 20 SMs).
-template <int D>
-static int fa_bwd_resident(int ctas) {
-  static const std::array<int, 9> table = [] {
-    std::array<int, 9> t{};
-    (void)cudaFuncSetAttribute(fa_bwd_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSmem<D>::kTotal);
-    for (int c = 1; c <= 8; ++c) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)c);
-      cfg.blockDim = dim3(kFbThreads);
-      cfg.dynamicSmemBytes = FbSmem<D>::kTotal;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)c;
-      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&t[c], fa_bwd_kernel<D, false>, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();
-        t[c] = c <= 2 ? sm_count() / c : 0;
-      }
-    }
-    return t;
-  }();
-  return table[ctas];
-}
-
 // CTAs per KV tile and head: as many as bring the longest walk (the first KV tile under a causal mask) down to an SM's share of all
 // steps; at least two steps each, eight where that makes more CTAs than SMs (a CTA's K and V loads and its dK / dV cost about one
 // and a half steps). They are two clusters of at most 8; where all CTAs would fit the SMs, the clusters are made small enough that
@@ -801,8 +773,9 @@ static int fa_bwd_splits(const pkb_attn_desc& d, int kv_tiles) {
   if (s > most / 2) s = most / 2;
   if (s < 2) return 1;
   int cluster = s < 16 ? (int)s / 2 : 8;
+  static const std::array<int, 9> resident = resident_clusters(fa_bwd_kernel<D, false>, kFbThreads, FbSmem<D>::kTotal);
   if (2 * cluster * kv_tiles * heads <= sms)
-    while (cluster > 1 && 2 * kv_tiles * heads > fa_bwd_resident<D>(cluster)) --cluster;
+    while (cluster > 1 && 2 * kv_tiles * heads > resident[cluster]) --cluster;
   return 2 * cluster;
 }
 

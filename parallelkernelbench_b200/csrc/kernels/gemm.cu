@@ -1,4 +1,5 @@
 // Host launchers of the tcgen05 GEMM (kernel template in pkb/gemm_umma.cuh).
+#include <array>
 #include <cstdlib>
 
 #include "pkb/api.h"
@@ -115,19 +116,25 @@ static int dispatch_pair(int epi, const CUtensorMap& ta, const void* b, long lon
   return kApiBadArgument;
 }
 
-// Up to 64 rows and at most one 128-column tile per SM: the kernel that shares a tile's K range between the CTAs of a cluster
-// (gemm_split.cuh). Measured against one CTA per tile, L2 flushed, us: 33 x 1024 x 8192 15.2 / 33.7, 7 x 264 x 16384 15.5 / 57.3,
-// 17 x 4096 x 14336 33.8 / 60.4, 1 x 14336 x 4096 33.7 / 44.0, 16 x 14336 x 4096 35.7 / 37.8, 64 x 256 x 256 9.2 / 9.2; with more
-// rows the exchange of 128-row partial sums costs what the shorter K range gives: 100 x 2048 x 2048 21.5 / 15.5.
-static bool split_fits(int M, int N) {
-  return M <= 64 && (N + 127) / 128 <= sm_count();
+// Up to 64 rows, at most one 128-column tile per SM and at least 24 K blocks: the kernel that shares a tile's K range between the CTAs of
+// a cluster (gemm_split.cuh). Measured against one CTA per tile, L2 flushed, us: 1 x 2048 x 2048 12.3 / 14.4, 64 x 2048 x 2048 13.8 / 14.4,
+// 33 x 1024 x 8192 14.4 / 32.8, 7 x 264 x 16384 16.2 / 56.6, 64 x 4096 x 4096 18.0 / 22.6; with one CTA per tile, where only the deeper ring
+// tells, 1 x 14336 x 4096 34.9 / 43.9, 16 x 14336 x 4096 34.8 / 36.4. Fewer K blocks: 1 x 1024 x 1024 10.3 / 10.3, 64 x 1024 x 1024 12.2 /
+// 11.6, 64 x 2048 x 512 12.2 / 10.1, 1 x 256 x 256 9.0 / 8.2. More than one tile per SM: 16 x 20000 x 4096 51.4 / 53.0, 64 x 128256 x 4096
+// 192 / 192, 128 rows of it 205 / 198 (1 row 182 / 242). More rows: 80 x 1024 x 8192 16.6 / 33.3 and 80 x 4096 x 4096 18.7 / 23.1, but 128 x
+// 2048 x 512 13.9 / 10.5 and 128 x 20000 x 4096 56 / 50.
+static bool split_fits(int M, int N, int K) {
+  return M <= 64 && (N + 127) / 128 <= sm_count() && K > 23 * kGemmBlockK;
 }
 
-// Cluster size: as many CTAs as leave every tile's cluster resident at once (a GPC holds 16 to 20 SMs: 16 clusters of 8, 32 of 4,
-// 64 of 2), and at least four K blocks each.
+// Cluster size: as many CTAs as leave every tile's cluster resident at once (15 clusters of 8 CTAs, 33 of 4, 74 of 2: a cluster stays
+// inside a group of 16 to 20 SMs), and at least four K blocks each. One cluster too many is a second wave: 64 x 2048 x 2048 (16 tiles)
+// 20.4 us on clusters of 8, 13.8 on 4.
+template <int EPI, bool OUT_F32, bool B_MN>
 static int split_count(int tiles, int num_k) {
-  int s = tiles <= 16 ? 8 : tiles <= 32 ? 4 : tiles <= 64 ? 2 : 1;
-  while (s > 1 && num_k < 4 * s) s >>= 1;
+  static const std::array<int, 9> resident = resident_clusters(gemm_split_kernel<EPI, OUT_F32, B_MN>, kGemmThreads, kSplitSmemTotal);
+  int s = 8;
+  while (s > 1 && (tiles > resident[s] || num_k < 4 * s)) s >>= 1;
   return s;
 }
 
@@ -143,7 +150,7 @@ static int launch_split(const void* a, long long lda, const void* b, long long l
             : encode_tmap_2d(&tb, kTmapBf16, b, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldb * 2, kGemmBlockK, kSplitBN, kSwizzle128);
   if (rc) return rc;
   const int tiles = (p.N + kSplitBN - 1) / kSplitBN;
-  const int splits = split_count(tiles, (p.K + kGemmBlockK - 1) / kGemmBlockK);
+  const int splits = split_count<EPI, OUT_F32, B_MN>(tiles, (p.K + kGemmBlockK - 1) / kGemmBlockK);
   auto kern = gemm_split_kernel<EPI, OUT_F32, B_MN>;
   PKB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemTotal));
   cudaLaunchConfig_t cfg = {};
@@ -249,7 +256,7 @@ extern "C" int pkb_gemm_bf16(const void* a, long long lda, const void* b, long l
 extern "C" int pkb_gemm_bf16_auto(const void* a, long long lda, const void* b, long long ldb, void* c, long long ldc, int M, int N,
                                   int K, const void* bias, float alpha, int epilogue, int out_f32, void* stream) {
   PKB_CHECK_ARG(M > 0 && N > 0 && K > 0, "empty problem");
-  if (!split_fits(M, N))
+  if (!split_fits(M, N, K))
     return M >= 512 && N >= 256 ? pkb_gemm_bf16_pair(a, lda, b, ldb, c, ldc, M, N, K, bias, alpha, epilogue, out_f32, 0, stream)
                                 : pkb_gemm_bf16(a, lda, b, ldb, c, ldc, M, N, K, bias, alpha, epilogue, out_f32, 0, 0, stream);
   PKB_CHECK_ARG(lda % 8 == 0 && ldb % 8 == 0 && K % 8 == 0, "lda, ldb, K must be multiples of 8");
@@ -417,7 +424,7 @@ extern "C" int pkb_gemm_bf16_bkn(const void* a, long long lda, const void* b, lo
   int ctas = sm_count();
   if (ctas > tiles) ctas = tiles;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (split_fits(M, N)) {
+  if (split_fits(M, N, K)) {
     p.kernel_id = 109;
     if (epilogue == kEpiSilu)
       return out_f32 ? launch_split<kEpiSilu, true, true>(a, lda, b, ldb, p, s) : launch_split<kEpiSilu, false, true>(a, lda, b, ldb, p, s);

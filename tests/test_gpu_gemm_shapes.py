@@ -23,7 +23,9 @@ def _check_gemm(y, a, w, bias=None, act="none"):
     assert (err <= bound).all(), f"{(err - bound).max().item():.3g} beyond the bound"
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 264, 64), (16, 128, 4096), (17, 8192, 520), (33, 1024, 1032), (64, 2048, 2048), (65, 136, 264),
+# among them K just below and above the limit of 24 blocks, and tiles at and beyond one wave of clusters of 8 (15), 4 (33) and 2 (74)
+@pytest.mark.parametrize("M,N,K", [(40, 1024, 1472), (40, 1024, 1480), (9, 1920, 2048), (64, 2048, 2048), (20, 4224, 1544), (20, 4232, 1544), (3, 9472, 1544),
+                                    (3, 9480, 1544), (1, 264, 64), (16, 128, 4096), (17, 8192, 520), (33, 1024, 1032), (65, 136, 264),
                                     (48, 18944, 64), (2, 18952, 136), (31, 72, 16384), (64, 8200, 8)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 def test_gemm_with_few_rows(M, N, K, out_dtype):

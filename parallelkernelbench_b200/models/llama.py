@@ -67,7 +67,7 @@ def rope_tables(cfg: LlamaConfig, device, dtype=torch.bfloat16):
 
 
 # =================================================================================================
-# one decoder layer on PyTorch library ops (impl="torch"); impl="ours" is ops.decoder.DecoderLayer
+# one decoder layer, on PyTorch library ops (impl="torch") or as one native call each way (impl="ours", ops.decoder.DecoderLayer)
 # =================================================================================================
 def _rot_half(x, cos, sin):
     h = x.shape[-1] // 2
@@ -79,8 +79,46 @@ def _rms_torch(x, g, eps):
     return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps) * g.float().reshape(-1)).to(x.dtype)
 
 
-def layer_forward(cfg: LlamaConfig, p: dict, x: torch.Tensor, cos, sin) -> torch.Tensor:
-    """``x`` is ``[S, hidden]`` (one sequence). ``p`` maps parameter names to bf16 tensors."""
+class _NativeLayer(torch.autograd.Function):
+    """A decoder layer with a tape, for programs that differentiate through :func:`layer_forward` themselves."""
+
+    @staticmethod
+    def forward(ctx, cfg, x, cos, sin, *params):
+        from ..ops.decoder import DecoderLayer
+
+        if any(t.dtype != torch.bfloat16 for t in (x, *params)):
+            raise TypeError("the native layer takes bf16 tensors")
+        for (name, shape), t in zip(cfg.layer_shapes(), params):
+            if t.numel() != shape[0] * shape[1]:
+                raise ValueError(f"{name} must have {shape[0]} x {shape[1]} elements, got {tuple(t.shape)}")
+        S, d = x.shape[0], cfg.head_dim
+        cos, sin = (t.to(torch.bfloat16).contiguous() for t in (cos, sin))
+        if x.shape[1] != cfg.hidden or cos.numel() != S * d or sin.numel() != S * d:
+            raise ValueError("x must be [S, hidden], cos and sin one row of head_dim values per token")
+        layer = DecoderLayer(S, cfg.hidden, cfg.ffn, cfg.heads, cfg.kv_heads, d, cfg.eps, 1.0 / math.sqrt(d))
+        flat = torch.cat([t.reshape(-1) for t in params])
+        x = x.contiguous()
+        x = x if x.data_ptr() % 16 == 0 else x.clone()
+        out, saved = layer.forward(x, flat, cos, sin, torch.empty(layer.fwd_scratch_bytes, dtype=torch.uint8, device=x.device))
+        ctx.save_for_backward(x, flat, cos, sin, saved)
+        ctx.layer, ctx.shapes = layer, [t.shape for t in params]
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        x, flat, cos, sin, saved = ctx.saved_tensors
+        dout = dout.contiguous()
+        dout = dout if dout.data_ptr() % 16 == 0 else dout.clone()
+        dflat = torch.empty_like(flat)
+        dx = ctx.layer.backward(x, flat, cos, sin, saved, dout, dflat, torch.empty(ctx.layer.bwd_scratch_bytes, dtype=torch.uint8, device=x.device))
+        grads = [g.view(s) for g, s in zip(dflat.split([s.numel() for s in ctx.shapes]), ctx.shapes)]
+        return None, dx, None, None, *grads
+
+
+def layer_forward(cfg: LlamaConfig, p: dict, x: torch.Tensor, cos, sin, impl: str = "torch") -> torch.Tensor:
+    """``x`` is ``[S, hidden]`` (one sequence). ``p`` maps parameter names to bf16 tensors. Differentiable in both."""
+    if impl == "ours":
+        return _NativeLayer.apply(cfg, x, cos, sin, *(p[name] for name, _ in cfg.layer_shapes()))
     S, d, Hq, Hkv = x.shape[0], cfg.head_dim, cfg.heads, cfg.kv_heads
     qkv = F.linear(_rms_torch(x, p["norm1"], cfg.eps), p["wqkv"])
     q = qkv[:, :Hq * d].reshape(1, S, Hq, d)

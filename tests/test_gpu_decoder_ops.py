@@ -289,3 +289,25 @@ def test_decoder_layer_against_autograd(S, H, Fn, hq, hkv, d):
     for got, want in ((out, ref.detach()), (dx, xr.grad), (dflat, fr.grad)):
         assert torch.isfinite(got).all()
         assert float((got.double() - want).norm() / want.norm()) < 1.5e-2
+
+
+def test_layer_forward_on_the_native_layer():
+    """Both implementations behind the one entry point, with gradients to the separate parameters."""
+    from parallelkernelbench_b200.models.llama import LlamaConfig, layer_forward, rope_tables, split_layer_params
+
+    cfg = LlamaConfig(layers=1, hidden=256, ffn=384, heads=4, kv_heads=2, vocab=64, seq=70)
+    flat = torch.randn(cfg.layer_numel(), device="cuda", generator=_gen(1)) * 0.05
+    flat[-512:] = 1 + flat[-512:]
+    x, dout = (torch.randn(70, 256, device="cuda", generator=_gen(s)).to(torch.bfloat16) for s in (2, 3))
+    cos, sin = rope_tables(cfg, "cuda")
+    res = []
+    for impl, dtype in (("ours", torch.bfloat16), ("torch", torch.float64)):
+        p = {k: v.detach().clone().requires_grad_() for k, v in split_layer_params(cfg, flat.to(torch.bfloat16).to(dtype)).items()}
+        xi = x.detach().to(dtype).requires_grad_()
+        with torch.nn.attention.sdpa_kernel(torch.nn.attention.SDPBackend.MATH):
+            out = layer_forward(cfg, p, xi, cos.to(dtype), sin.to(dtype), impl)
+            out.backward(dout.to(dtype))
+        res.append([out.detach(), xi.grad, *(p[k].grad for k in p)])
+    for got, want in zip(*res):
+        assert got.shape == want.shape
+        assert float((got.double() - want).norm() / want.norm()) < 1.5e-2      # as for the layer itself

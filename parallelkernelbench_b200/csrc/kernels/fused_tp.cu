@@ -464,17 +464,20 @@ int pkb_tp_ag_gemm_set_wait_stats(void* dev_words) {
   return kApiOk;
 }
 
-// Default number of communication CTAs of the all-gather -> GEMM kernel for a group of `world` ranks (bulk_push: the TMA bulk
-// ring; otherwise the thread-copy push). Exposed so that the rule can be checked without a GPU.
 // Width of the CTA pairs' tiles: 128 columns where tiles of 256 would leave half of the pairs without one (the same on every
-// rank: it follows from the shapes alone).
+// rank: it follows from the shapes alone). At one rank, us on 256 / 128 columns, by the number of 256-wide tiles: GEMM 1 16 tiles 44.0 / 30.2,
+// 32 69.7 / 53.1 (256 x 8192 x 8192), 40 52.0 / 48.1, 64 48.1 / 42.0, 96 60.4 / 48.4, 160 75.7 / 66.5; GEMM 2 16 tiles 44.2 / 37.8, 32 76.8 /
+// 64.5, 36 73.1 / 61.4, 40 60.6 / 75.8 and 86.4 / 91.7, 64 63.5 / 79.3. The line is GEMM 2's; GEMM 1 would gain beyond it.
 static int tp_tile_n(int M, int N) {
   const long long tiles = (long long)((M + kGemm2TileM - 1) / kGemm2TileM) * ((N + 255) / 256);
   return 4 * tiles <= sm_count() ? 128 : 256;
 }
 
+// Default number of communication CTAs of the all-gather -> GEMM kernel for a group of `world` ranks (bulk_push: the TMA bulk
+// ring; otherwise the thread-copy push). Exposed so that the rule can be checked without a GPU. A rank by itself has nobody to push
+// to: no communication CTAs, no barrier.
 extern "C" int pkb_tp_default_comm_ctas(int world, int bulk_push) {
-  if (world <= 1) return 2;
+  if (world <= 1) return 0;
   if (bulk_push) return world >= 8 ? 16 : (world > 4 ? 12 : 8);
   return world >= 8 ? 16 : 8;
 }
@@ -557,8 +560,7 @@ int pkb_tp_ag_gemm(const pkb_symm_ctx* h, const void* x_local, int rows, int K,
   // producers wait 169 us per call for 96 MiB of remote rows, 8 CTAs 2 us), and the GEMM consumes one remote shard per
   // 1/W of its run time, so the rate the push needs grows with W while the shard size stays: 8 CTAs cover a 32 MiB shard in
   // 115 us, which is enough up to 4 ranks (175 us per shard of GEMM time) and not at 8 ranks (87 us), where 16 are used.
-  // A rank by itself has nobody to push to: no communication CTAs, no barrier.
-  if (comm_ctas <= 0) comm_ctas = W == 1 ? 0 : pkb_tp_default_comm_ctas(W, a.bulk_push);
+  if (comm_ctas <= 0) comm_ctas = pkb_tp_default_comm_ctas(W, a.bulk_push);
   comm_ctas = (comm_ctas + 1) & ~1;  // whole clusters
   const int sms = sm_count() & ~1;
   PKB_CHECK_ARG(comm_ctas < sms && comm_ctas <= kSymmMaxBlocks, "too many communication CTAs");

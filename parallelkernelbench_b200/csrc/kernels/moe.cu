@@ -78,7 +78,8 @@ __global__ void moe_plan_kernel(const int* __restrict__ all_counts, int world, i
 
 // Softmax over up to 256 experts and top-k selection, one warp per token. Lane l holds experts l, l + 32, ...
 // Selection = k rounds of a warp-wide arg-max on (probability, lower index wins ties), so the output is sorted by
-// descending probability like torch.topk. The histogram is accumulated per block in shared memory first.
+// descending probability like torch.topk. A NaN logit has probability 0 (a token with nothing else has gates NaN), so that every round
+// finds an expert. The histogram is accumulated per block in shared memory first.
 constexpr int kRouteMaxPerLane = 8;
 
 // work: NULL (counts holds zeros and is added to), or int32 [E + 1] that is zero before and after the kernel: counts is then
@@ -115,7 +116,7 @@ moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __
     float sum = 0.f;
 #pragma unroll
     for (int j = 0; j < kRouteMaxPerLane; ++j) {
-      v[j] = (j * 32 + lane) < num_experts ? expf(v[j] - m) : -1.f;   // probabilities are >= 0: -1 marks "absent / taken"
+      v[j] = (j * 32 + lane) < num_experts ? fmaxf(expf(v[j] - m), 0.f) : -1.f;   // probabilities are >= 0: -1 marks "absent / taken"
       sum += fmaxf(v[j], 0.f);
     }
     sum = warp_sum(sum);

@@ -57,6 +57,28 @@ def test_quantising_dispatch_matches_quantise_then_copy(group, T, hidden, E, k, 
     group.heap.release(mark)
 
 
+@pytest.mark.parametrize("E,k", [(8, 2), (40, 8), (256, 8)])
+def test_routing_of_logits_that_are_not_numbers(E, k):
+    """Every assignment goes to an expert that exists, k different ones a token; rows without such logits are as they were."""
+    from parallelkernelbench_b200.ops.moe import route_topk
+
+    logits = torch.randn(9, E, device="cuda", generator=torch.Generator(device="cuda").manual_seed(E))
+    want = route_topk(logits, None, k)
+    bad = logits.clone()
+    bad[1] = float("nan")
+    bad[2, :E - 1] = float("nan")                                         # one number is left
+    bad[3, 5] = float("nan")
+    bad[4, 3] = float("inf")
+    bad[5] = float("-inf")
+    gates, idx, counts = route_topk(bad, None, k)
+    assert ((idx >= 0) & (idx < E)).all() and int(counts.sum()) == 9 * k
+    assert all(row.unique().numel() == k for row in idx)
+    assert torch.equal(counts, torch.bincount(idx.view(-1).long(), minlength=E).int())
+    for r in (0, 6, 7, 8):
+        assert torch.equal(idx[r], want[1][r]) and torch.equal(gates[r], want[0][r])
+    assert gates[1].isnan().all() and idx[1].tolist() == list(range(k)) and int(idx[2, 0]) == E - 1
+
+
 def test_conversion_of_received_rows_leaves_own_rows_alone():
     """What a rank of a larger group does after the dispatch: rows of its own segment are bf16 already."""
     from parallelkernelbench_b200 import _native as nv

@@ -23,8 +23,8 @@ template <int BN, bool B_MN>
 struct Gemm2Tile {
   static_assert(BN == 256 || BN == 192 || BN == 128, "tile widths of the CTA-pair kernel");
   static constexpr int kStages = BN == 128 ? 8 : kGemm2Stages;
-  // an MN-major B comes in 64-column boxes: at BN = 192 half of the second box is not used
-  static constexpr int kBoxesMn = (BN / 2 + 63) / 64;
+  static_assert(!B_MN || BN % 128 == 0, "an MN-major B comes in boxes of 64 columns");
+  static constexpr int kBoxesMn = BN / 128;
   static constexpr int kBBytes = B_MN ? kBoxesMn * 8192 : BN / 2 * kGemmBlockK * 2;
   static constexpr int kStageBytes = kGemm2ABytes + kBBytes;
   static_assert(kStages * kStageBytes <= kGemm2Stages * kGemm2StageBytes, "the ring outgrew the shared-memory plan");

@@ -50,7 +50,6 @@ struct FaBwdParams {
   pkb_attn_desc d;
   const float* lse2;    // [batch, hq, sq]  log-sum-exp in base-2 units
   const float* delta;   // [batch, hq, sq]  rowsum(dO * O)
-  float* dq;            // [batch * sq, hq, D] fp32, zeroed by the kernel before
   float* dk;            // [batch * skv, hkv, D] fp32
   float* dv;            // [batch * skv, hkv, D] fp32
   // Context-parallel form: when seg_scatter != 0 the dK / dV rows of KV segment s are ADDED (fp32 vector reductions) into
@@ -836,7 +835,6 @@ static int launch_fa_bwd(const pkb_attn_desc& d, const void* q, const void* k, c
   p.d = d;
   p.lse2 = static_cast<const float*>(lse2);
   p.delta = static_cast<const float*>(delta);
-  p.dq = static_cast<float*>(dq);
   p.dk = static_cast<float*>(dk);
   p.dv = static_cast<float*>(dv);
   p.splits = splits;

@@ -90,7 +90,7 @@ struct BwdScratch {
     lse2 = c.take(S * L.hq * 4);
     dq_elems = S * qd;
     dk_elems = S * kd;
-    dqkv32 = c.take((dq_elems + 2 * dk_elems) * 4);      // dq, dk, dv in one piece: one fill
+    dqkv32 = c.take((dq_elems + 2 * dk_elems) * 4);      // dq, dk, dv
     dqkv = c.take(S * (qd + 2 * kd) * 2);
     dh = c.take(S * L.hidden * 2);
     partial = c.take((long long)pkb_rmsnorm_bwd_partials(L.tokens, L.hidden) * L.hidden * 4);

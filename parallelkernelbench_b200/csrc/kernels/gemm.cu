@@ -46,8 +46,10 @@ static bool pair_mn_enabled() {
 // Tile width of the CTA-pair kernel. A wave is sm_count / 2 tiles of 256 x BN, so a problem costs its number of waves times the
 // width, times a factor for narrow tiles, which read more operand bytes per flop. The factors are measured (us at 256 / 192 /
 // 128): 1333 x 4104 x 4096 (2, 2, 3 waves) 51.9 / 43.8 / 46.0; 4096 x 4096 x 4096 (4, 5, 7) 94.2 / 94.1 / 94.2; 4104 x 4096 x 1336
-// (4, 6, 8) 50 / 56 / 64. With an MN-major B narrow tiles gain less (half of a 64-column box is not used at 192): 1333 x 4104 x
-// 4096 51.2 / 49.2 / 47.1, 1333 x 4096 x 4104 51.2 / 57.3 / 59.4, 4104 x 4096 x 1336 41.8 / 56.1 / 54.2.
+// (4, 6, 8) 50 / 56 / 64. With an MN-major B what narrow tiles gain does not follow from the waves (256 / 128: 1333 x 4104 x 4096 52.2 /
+// 48.1, 1536 x 4096 x 14336 150 / 128, but 1333 x 4096 x 4104 52.2 / 59.4, 1333 x 14336 x 4096 114 / 123), so 128 columns are taken only where
+// they save 30 % of the columns computed (512 x 4096 x 4096 29.7 / 23.5, 640 x 2048 x 8192 50.3 / 33.8); 192 columns, of which half a box is
+// not used, can never save as many.
 static int pair_tile_n(int M, int N, int pairs, bool b_mn) {
   const long long num_m = (M + 255) / 256;
   auto cost = [&](int bn, double per_col) {
@@ -56,7 +58,7 @@ static int pair_tile_n(int M, int N, int pairs, bool b_mn) {
   };
   int best = 256;
   double c = cost(256, 1.0);
-  if (cost(192, b_mn ? 1.4 : 1.09) < c) { best = 192; c = cost(192, b_mn ? 1.4 : 1.09); }
+  if (!b_mn && cost(192, 1.09) < c) { best = 192; c = cost(192, 1.09); }
   if (cost(128, b_mn ? 1.4 : 1.16) < c) best = 128;
   return best;
 }
@@ -99,7 +101,9 @@ static int launch_pair(const CUtensorMap& ta, const void* b, long long ldb, Gemm
                 : encode_tmap_2d(&tb, kTmapBf16, b, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldb * 2, kGemmBlockK, (uint32_t)bn / 2, kSwizzle128);
   if (rc) return rc;
   if (bn == 128) return launch_pair_bn<EPI, OUT_F32, A_MN, B_MN, 128>(ta, tb, p, ctas, stream);
-  if (bn == 192) return launch_pair_bn<EPI, OUT_F32, A_MN, B_MN, 192>(ta, tb, p, ctas, stream);
+  if constexpr (!B_MN) {
+    if (bn == 192) return launch_pair_bn<EPI, OUT_F32, A_MN, B_MN, 192>(ta, tb, p, ctas, stream);
+  }
   return launch_pair_bn<EPI, OUT_F32, A_MN, B_MN, 256>(ta, tb, p, ctas, stream);
 }
 

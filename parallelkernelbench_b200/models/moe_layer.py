@@ -1,10 +1,11 @@
 """Expert-parallel MoE layer: router -> fp8 dispatch -> grouped SwiGLU expert FFN -> combine.
 
-Five of our kernels per forward besides the router: histogram, plan, dispatch (P2P push of fp8 rows
-with 1x128 scales), two grouped tcgen05 GEMMs (gate/up with the SwiGLU epilogue, then down, writing
-into the symmetric buffer the combine reads), combine (P2P pull, gate-weighted, deterministic order).
-The router GEMM runs on the dense tcgen05 kernel; softmax and top-k over a few hundred experts are
-PyTorch ops. ``push_combine`` moves the way home into the down GEMM: the dispatch delivers (sender, assignment index) with every row, the
+Six launches per forward on one rank: the router GEMM (dense tcgen05 kernel), routing (softmax, top-k, histogram, and in its last
+block the plan), dispatch (P2P push of rows, quantised to e4m3 with 1x128 scales on the way), two grouped tcgen05 GEMMs (gate/up
+with the SwiGLU epilogue, then down, writing into the symmetric buffer the combine reads), combine (P2P pull, gate-weighted,
+deterministic order). With more ranks the counts are gathered and the plan is a launch of its own, and fp8 rows from other ranks
+are converted after the dispatch where the experts take bf16. More than 256 experts, or ``fused_router=False``: softmax and top-k
+as PyTorch ops and a histogram launch. ``push_combine`` moves the way home into the down GEMM: the dispatch delivers (sender, assignment index) with every row, the
 GEMM's epilogue stores each output row straight into the sender's buffer over NVLink, and the combine kernel only reads local
 memory after its barrier.
 Reference behaviour: reference/31_fused_moe_fwd.py:254-315 (with shared expert weights;
@@ -72,6 +73,8 @@ class EPMoELayer:
         return gemm_bf16(x, self.w_router, out_dtype=torch.float32, mode="single", block_n=128)
 
     def route(self, x: torch.Tensor):
+        """Gates and experts of every token ``([T, k], [T, k])``, without the plan: for callers that look at the routing, or plan
+        themselves (``forward`` has both in one launch)."""
         logits = self._logits(x)
         if self.cfg.fused_router:
             gates, idx, _ = route_topk(logits, self.router_bias_f32, self.cfg.top_k, counts=self.ex.counts)
